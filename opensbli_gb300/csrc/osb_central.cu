@@ -2,6 +2,7 @@
 // once per precision (OSB_CENTRAL_T).
 #include "osb_closures.h"
 #include "osb_internal.h"
+#include "osb_central64.cuh"
 
 #include <algorithm>
 #include <cmath>
@@ -12,13 +13,9 @@ namespace {
 // Faces whose central derivatives take the one-sided closures (ModifyCentralDerivative walls).
 inline bool is_wall(int kind) { return kind == OSB_BC_ISOTHERMAL_WALL || kind == OSB_BC_ADIABATIC_WALL; }
 
-template <typename T, int CONV, int VISC, bool FUSE, int CY, bool BULK, bool WALL = false>
-int launch_central_k(osb_ctx* c, Block& bl, int first, const RkFuse& rf) {
-  using Fd = CentralFields<T, CONV, VISC>;
-  size_t smem = (size_t)Fd::N * CRING * CTile<CY, WALL ? 4 : CH>::CPL * sizeof(T);
-  if (BULK) smem += CTile<CY>::RAW * sizeof(float) + 2 * sizeof(unsigned long long);
-  auto kern = k_central3d<T, CONV, VISC, FUSE, CY, BULK, WALL>;
-  OSB_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+// Constants of one block's central terms; WALL: with the closures at its wall faces.
+template <bool WALL>
+CentralParams central_params(const Block& bl) {
   CentralParams cp{};
   const osb_block_desc& d = bl.d;
   cp.gama = d.gama;
@@ -59,6 +56,17 @@ int launch_central_k(osb_ctx* c, Block& bl, int first, const RkFuse& rf) {
         cp.c2f[r][m] = (float)cl.c2[r][m];
       }
   }
+  return cp;
+}
+
+template <typename T, int CONV, int VISC, bool FUSE, int CY, bool BULK, bool WALL = false>
+int launch_central_k(osb_ctx* c, Block& bl, int first, const RkFuse& rf) {
+  using Fd = CentralFields<T, CONV, VISC>;
+  size_t smem = (size_t)Fd::N * CRING * CTile<CY, WALL ? 4 : CH>::CPL * sizeof(T);
+  if (BULK) smem += CTile<CY>::RAW * sizeof(float) + 2 * sizeof(unsigned long long);
+  auto kern = k_central3d<T, CONV, VISC, FUSE, CY, BULK, WALL>;
+  OSB_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const CentralParams cp = central_params<WALL>(bl);
   const BlockK& k = bl.k;
   // z chunks per column: whole waves of resident CTAs; a chunk starts by staging four planes
   // (two of halo) at about a third of the cost of a computed plane each
@@ -77,7 +85,7 @@ int launch_central_k(osb_ctx* c, Block& bl, int first, const RkFuse& rf) {
 // Tile height of the FP32 kernels: 8 rows unless the ring holds the KGP form's eleven fields of a
 // block whose cross-section already gives every SM several columns (measured: 8 rows are 37 %
 // faster on the 64^3 central TGV and equal on the 256^3 TENO5 one; 4 rows are 1.4 % faster for
-// the 256^3 KGP form).  The FP64 kernels (FP64-pipe bound, a ring twice as large) keep 4 rows.
+// the 256^3 KGP form).  FP64 (the KGP form alone, FP64-pipe bound, a ring twice as large): 4 rows.
 template <typename T, int CONV, int VISC, bool FUSE, bool BULK>
 int launch_central_h(osb_ctx* c, Block& bl, int first, const RkFuse& rf) {
   if constexpr (CONV == 0 && !BULK) {
@@ -91,16 +99,42 @@ int launch_central_h(osb_ctx* c, Block& bl, int first, const RkFuse& rf) {
   return OSB_OK;
 }
 
+// FP64 blocks without wall faces: Feiereisen and viscous terms (k_central_f64).
+template <int CONV, int VISC>
+int launch_central_f64(osb_ctx* c, Block& bl, int first) {
+  auto kern = k_central_f64<CONV, VISC>;
+  constexpr size_t smem = c64_smem<CONV, VISC>();
+  OSB_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const BlockK& k = bl.k;
+  const long cols = (long)((k.n[0] + CX - 1) / CX) * ((k.n[1] + C64Y - 1) / C64Y);
+  const long slots = (long)resident_ctas(kern, C64T, smem) * c->sm_count;
+  // a chunk's four planes of start-up cost their staging, about a fifth of a computed plane each
+  const int nz = wave_chunks(k.n[2], cols, slots, 0.9, 4);
+  const int czc = (k.n[2] + nz - 1) / nz;
+  dim3 grid((k.n[0] + CX - 1) / CX, (k.n[1] + C64Y - 1) / C64Y, (k.n[2] + czc - 1) / czc);
+  timing_begin(c, FAM_CENTRAL);
+  kern<<<grid, C64T, smem, c->stream>>>(k, central_params<false>(bl), first, czc);
+  timing_end(c);
+  c->launches++;
+  return OSB_OK;
+}
+
 // With rf (FP32 path) the kernel applies the RK update instead of storing the residual; its
 // planes come in by register loads or, after osb_set_central_staging(1), by bulk copies.
 template <typename T, int CONV, int VISC>
 int launch_central_t(osb_ctx* c, Block& bl, int first, const RkFuse* rf) {
-  if constexpr (sizeof(T) == 4) {
-    const bool wall = is_wall(bl.d.bc[1][0]) || is_wall(bl.d.bc[1][1]);
-    if (rf && c->central_bulk && !wall) return launch_central_h<T, CONV, VISC, true, true>(c, bl, first, *rf);
-    if (rf) return launch_central_h<T, CONV, VISC, true, false>(c, bl, first, *rf);
+  const bool wall = is_wall(bl.d.bc[1][0]) || is_wall(bl.d.bc[1][1]);
+  if constexpr (sizeof(T) == 8 && CONV != 2) {
+    if (!wall) return launch_central_f64<CONV, VISC>(c, bl, first);
+    if constexpr (CONV == 0) return launch_central_k<T, 0, VISC, false, 4, false, true>(c, bl, first, RkFuse{});
+    return fail(OSB_ENOTSUP, "walls are implemented for shock-capturing schemes");
+  } else {
+    if constexpr (sizeof(T) == 4) {
+      if (rf && c->central_bulk && !wall) return launch_central_h<T, CONV, VISC, true, true>(c, bl, first, *rf);
+      if (rf) return launch_central_h<T, CONV, VISC, true, false>(c, bl, first, *rf);
+    }
+    return launch_central_h<T, CONV, VISC, false, false>(c, bl, first, RkFuse{});
   }
-  return launch_central_h<T, CONV, VISC, false, false>(c, bl, first, RkFuse{});
 }
 
 template <typename T>

@@ -26,13 +26,12 @@ template <typename T, int ND, int D, int SCH, int AVG, bool CURV, bool FUSE, int
 int launch_sweep_k(osb_ctx* c, const BlockK& k, const SchemeParams& sp, int N, int other, const RkFuse& rf) {
   auto kern = k_flux_sweep<T, ND, D, SCH, AVG, CURV, FUSE, FLX>;
   const long slots = (long)resident_ctas(kern, SWEEP_THREADS, 0) * c->sm_count;
-  const long gx = (k.n[0] + SWEEP_THREADS - 1) / SWEEP_THREADS;
-  int nseg = wave_chunks(N, gx * other, slots, 1.5, 8);
+  const long gx = ((long)k.n[0] * other + SWEEP_THREADS - 1) / SWEEP_THREADS;
+  int nseg = wave_chunks(N, gx, slots, 1.5, 8);
   const int seg = (N + nseg - 1) / nseg;
   nseg = (N + seg - 1) / seg;
-  const long gy = (long)other * nseg;
-  dim3 grid((unsigned)gx, (unsigned)std::min(gy, 65535L), (unsigned)((gy + 65534) / 65535));
-  if (grid.z > 1) return fail(OSB_ENOTSUP, "block too large for the sweep grid");
+  if (other > 65535 || nseg > 65535) return fail(OSB_ENOTSUP, "block too large for the sweep grid");
+  dim3 grid((unsigned)gx, (unsigned)nseg);
   kern<<<grid, SWEEP_THREADS, 0, c->stream>>>(k, sp, seg, nseg, 0, rf);
   return OSB_OK;
 }

@@ -352,17 +352,21 @@ __device__ __forceinline__ int gvar(int lv) {
 }
 
 // ---------------------------------------------------------------------------------------
-// Sweep along y (D=1) or z (D=2): thread = (x, transverse, segment).
+// Sweep along y (D=1) or z (D=2): thread = (line, segment), lines numbered along x first.
 // The fields of point j+3 and the residual of point j that iteration j needs are copied with
 // cp.async into a per-thread ring of shared-memory slots one iteration ahead, so their latency
 // overlaps a whole interface's arithmetic without holding registers (the register file is the
 // occupancy limit of these kernels).  A slot is refilled two iterations after it was read.
+// FP32: three CTAs per SM (168 registers).  The packed flux wants independent pairs in flight more
+// than warps: 256^3 TENO5 y sweep 0.59 ms with 12 warps per SM, 0.62 with 16 at 128 registers, 0.78
+// with 20 (spilling); 0.79 before the packed flux.  The curvilinear z sweep of the 4-block case
+// takes 0.22 ms instead of 0.29.
 constexpr int SWEEP_THREADS = 128, SWEEP_RING = 3;
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_prev() { asm volatile("cp.async.wait_group 1;\n" ::: "memory"); }
 
 template <typename T, int ND, int D, int SCH, int AVG, bool CURV, bool FUSE, int FLX = 0>
-__global__ void __launch_bounds__(SWEEP_THREADS, sizeof(T) == 4 ? 4 : 1)
+__global__ void __launch_bounds__(SWEEP_THREADS, sizeof(T) == 4 ? 3 : 1)
     k_flux_sweep(BlockK b, SchemeParams spd, int seg, int nseg, int first, RkFuse rf) {
   constexpr int NV = ND + 2;
   constexpr int NF = SweepFields<ND, CURV>::N;
@@ -372,15 +376,12 @@ __global__ void __launch_bounds__(SWEEP_THREADS, sizeof(T) == 4 ? 4 : 1)
   __shared__ T ring[SWEEP_RING][NS][SWEEP_THREADS];
   const SP<T> sp(spd);
   const int tid = threadIdx.x;
-  const int x = blockIdx.x * blockDim.x + tid;
-  const int other = blockIdx.y / nseg, sidx = blockIdx.y % nseg;
-  if (x >= b.n[0]) return;
-  int c1 = 0, c2 = 0;
-  if (ND == 3) {
-    if (D == 1) c2 = other + blockIdx.z * 65535; else c1 = other + blockIdx.z * 65535;
-    if (D == 1 && c2 >= b.n[2]) return;
-    if (D == 2 && c1 >= b.n[1]) return;
-  }
+  // the block's lines (x, transverse) are one index space, so rows of any length fill the warps:
+  // with one row per CTA the 131 x 97 x 110 block left a fifth of the lanes and half of the CTAs idle
+  const int line = blockIdx.x * SWEEP_THREADS + tid, sidx = blockIdx.y;
+  const int c3 = ND == 3 ? line / b.n[0] : 0, x = line - c3 * b.n[0];
+  const int c1 = ND == 3 && D == 2 ? c3 : 0, c2 = ND == 3 && D == 1 ? c3 : 0;
+  if (ND == 3 ? c3 >= b.n[D == 1 ? 2 : 1] : x >= b.n[0]) return;
   const int s = b.st[D];
   const int base = lin(b, x, c1, c2);
   const int N = b.n[D];
@@ -497,6 +498,8 @@ __global__ void __launch_bounds__(SWEEP_THREADS, sizeof(T) == 4 ? 4 : 1)
 // one window start; the length is chosen on the host (whole waves of resident CTAs) or fixed by
 // osb_set_variant.  Row pitches are odd, so the 32 lanes (rows) of a warp hit distinct banks.
 constexpr int XCH = 4, XRING = 2, XCOLS = XCH * XRING, XPITCH = XCOLS + 1, XOUT = 8, XOPITCH = XOUT + 1;
+// FP32: six CTAs of two warps per SM, 168 registers (256^3 TENO5: 0.61 ms; 0.76 with eight CTAs at
+// 128; 0.86 before the packed flux).
 constexpr int XWARPS = 2;
 
 template <typename T, int NF, int NO>
@@ -507,7 +510,7 @@ struct XTile {
 };
 
 template <typename T, int ND, int SCH, int AVG, bool CURV, int FLX = 0>
-__global__ void __launch_bounds__(32 * XWARPS) k_flux_x(BlockK b, SchemeParams spd, int first, int xseg,
+__global__ void __launch_bounds__(32 * XWARPS, sizeof(T) == 4 ? 6 : 1) k_flux_x(BlockK b, SchemeParams spd, int first, int xseg,
                                                          const int* __restrict__ xrows) {
   constexpr int NV = ND + 2;
   constexpr int NF = SweepFields<ND, CURV>::N;

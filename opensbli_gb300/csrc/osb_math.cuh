@@ -38,7 +38,7 @@ struct SchemeParams {
   // sweeps' register cap the compiler re-derives such values inside the loop instead of
   // keeping them in registers (measured: six FP64-pipe conversions per point in the FP32 y/z
   // sweeps, 34 % FP64-pipe activity)
-  float gama_f, g1_f, teno_eps_f, teno_ct_f, sfc_f, eps32_rel_f;
+  float gama_f, g1_f, ig1_f, teno_eps_f, teno_ct_f, sfc_f, eps32_rel_f;
 };
 
 __host__ __device__ inline SchemeParams scheme_params(double gama, double teno_eps, double teno_ct, double sfc,
@@ -50,6 +50,7 @@ __host__ __device__ inline SchemeParams scheme_params(double gama, double teno_e
   p.sfc = sfc;
   p.eps32_rel = eps32_rel;
   p.ig1 = 1.0 / (gama - 1.0);
+  p.ig1_f = (float)p.ig1;
   p.gama_f = (float)gama;
   p.g1_f = (float)(gama - 1.0);
   p.teno_eps_f = (float)teno_eps;
@@ -72,9 +73,9 @@ struct SP<double> {
 };
 template <>
 struct SP<float> {
-  float gama, g1, teno_eps, teno_ct, sfc, eps32_rel;
+  float gama, g1, ig1, teno_eps, teno_ct, sfc, eps32_rel;
   __device__ __forceinline__ explicit SP(const SchemeParams& p)
-      : gama(p.gama_f), g1(p.g1_f), teno_eps(p.teno_eps_f), teno_ct(p.teno_ct_f), sfc(p.sfc_f),
+      : gama(p.gama_f), g1(p.g1_f), ig1(p.ig1_f), teno_eps(p.teno_eps_f), teno_ct(p.teno_ct_f), sfc(p.sfc_f),
         eps32_rel(p.eps32_rel_f) {}
 };
 
@@ -470,9 +471,10 @@ __device__ __forceinline__ void make_pt(Pt<double, ND>& s, double gm) {
 //   P = E - u.m + |u|^2/2 rho,  D = m_n - u_n rho,
 //   entropy wave   e  = rho - (gama - 1) / a^2 P,
 //   vorticity      m_t2 - u_t2 rho  and  u_t1 rho - m_t1       (the rows times the average density)
-//   acoustic       P +- a / (gama - 1) D                       (the rows over their common factor)
-// and the projected flux of a point is its own u_n times that, plus p (u_n' - u_n) and
-// +- p a / (gama - 1) in the acoustic rows and -(gama - 1) / a^2 p (u_n' - u_n) in the entropy row.  A
+//   acoustic       (gama - 1) / a P +- D                       (the rows over their common factor)
+// and the projected flux of a point is its own u_n times that, plus (gama - 1) / a p (u_n' - u_n) +- p in
+// the acoustic rows (the pressure then reaches the momentum flux without a rounded factor) and
+// -(gama - 1) / a^2 p (u_n' - u_n) in the entropy row.  A
 // row's constant factor commutes with the reconstruction (its epsilon is scaled instead, ReconEps),
 // so neither it nor the 1/2 of the flux splitting is applied to the twelve values of a wave, and
 // 1D, 2D and 3D share the form: their rows differ by that factor alone.
@@ -487,7 +489,7 @@ __device__ __forceinline__ void char_flux_f64(const Pt<double, ND> (&w)[6], cons
   const double g1 = sp.g1;
   const Pt<double, ND>& L = w[2];
   const Pt<double, ND>& R = w[3];
-  double u[ND], a, a2, ia2, rho2;  // rho2: the average density squared
+  double u[ND], a, ia, rho2;  // rho2: the average density squared
   double ke = 0.0;
   if (AVG == AVG_ROE) {
     const double inv = rcp_newton(L.s + R.s), wl = L.s * inv, wr = R.s * inv;
@@ -496,10 +498,9 @@ __device__ __forceinline__ void char_flux_f64(const Pt<double, ND> (&w)[6], cons
       u[i] = wl * L.u[i] + wr * R.u[i];
       ke += u[i] * u[i];
     }
-    a2 = g1 * (wl * L.H + wr * R.H - 0.5 * ke);
-    const double ia = rsqrt(a2);
+    const double a2 = g1 * (wl * L.H + wr * R.H - 0.5 * ke);
+    ia = rsqrt(a2);
     a = a2 * ia;
-    ia2 = ia * ia;
     rho2 = L.q[0] * R.q[0];
   } else {
 #pragma unroll
@@ -508,12 +509,11 @@ __device__ __forceinline__ void char_flux_f64(const Pt<double, ND> (&w)[6], cons
       ke += u[i] * u[i];
     }
     a = 0.5 * (L.a + R.a);
-    a2 = a * a;
-    ia2 = rcp_newton(a2);
+    ia = rcp_newton(a);
     const double rho = 0.5 * (L.q[0] + R.q[0]);
     rho2 = rho * rho;
   }
-  const double hk = 0.5 * ke, g = g1 * ia2, ag = a * sp.ig1;
+  const double hk = 0.5 * ke, gi = g1 * ia, g = gi * ia;
   const double lam_u = sp.sfc * fmax(fabs(L.u[0]), fabs(R.u[0]));
   const double lam_p = sp.sfc * fmax(fabs(L.u[0] + L.a), fabs(R.u[0] + R.a));
   const double lam_m = sp.sfc * fmax(fabs(L.u[0] - L.a), fabs(R.u[0] - R.a));
@@ -576,28 +576,28 @@ __device__ __forceinline__ void char_flux_f64(const Pt<double, ND> (&w)[6], cons
     t2 = 0.5 * wave(fp, fm, 4.0 * rho2);
   }
   // acoustic waves
-  const double s2a = ND == 1 ? 16.0 * (a2 * sp.ig1) * (a2 * sp.ig1) : 8.0 * rho2 * (ag * ag);
+  const double s2a = ND == 1 ? 16.0 * a * a : 8.0 * rho2;
 #pragma unroll
   for (int m = 0; m < 6; ++m) {
-    const double c = __fma_rn(ag, D[m], P[m]);
-    const double f = __fma_rn(w[m].u[0], c, __fma_rn(w[m].p, ag, W[m]));
+    const double c = __fma_rn(gi, P[m], D[m]);
+    const double f = __fma_rn(w[m].u[0], c, __fma_rn(gi, W[m], w[m].p));
     fp[m] = __fma_rn(lam_p, c, f);
     fm[m] = __fma_rn(-lam_p, c, f);
   }
   const double rp = wave(fp, fm, s2a);
 #pragma unroll
   for (int m = 0; m < 6; ++m) {
-    const double c = __fma_rn(-ag, D[m], P[m]);
-    const double f = __fma_rn(w[m].u[0], c, __fma_rn(-w[m].p, ag, W[m]));
+    const double c = __fma_rn(gi, P[m], -D[m]);
+    const double f = __fma_rn(w[m].u[0], c, __fma_rn(gi, W[m], -w[m].p));
     fp[m] = __fma_rn(lam_m, c, f);
     fm[m] = __fma_rn(-lam_m, c, f);
   }
   const double rm = wave(fp, fm, s2a);
   // back to physical space
-  const double h = 0.25 * g, A = h * (rp + rm), B = h * a * (rp - rm), F0 = r0 + A;
+  const double S = 0.25 * (rp + rm), B = 0.25 * (rp - rm), F0 = __fma_rn(ia, S, r0);
   fh[0] = F0;
   fh[1] = __fma_rn(u[0], F0, B);
-  double e = __fma_rn(hk, F0, __fma_rn(a2 * sp.ig1, A, u[0] * B));
+  double e = __fma_rn(hk, F0, __fma_rn(a * sp.ig1, S, u[0] * B));
   if constexpr (ND >= 2) {
     fh[2] = __fma_rn(u[1], F0, -t2);
     e = __fma_rn(-u[1], t2, e);
@@ -609,6 +609,199 @@ __device__ __forceinline__ void char_flux_f64(const Pt<double, ND> (&w)[6], cons
   fh[NV - 1] = e;
 }
 
+// ---------------------------------------------------------------------------------------
+// FP32 characteristic flux on packed pairs.
+//
+// The FP32 sweeps are bound by instruction issue (81-83 % of the issue slots, the FMA pipe 65-68 %
+// busy: profiles/kernels_tgv256_teno5_fp32.md).  sm_103a's packed FP32 instructions (fma / mul / add
+// on a float2) do two lanes' work in one issue slot at the same FMA-pipe time, so the reconstruction
+// runs on pairs that share every coefficient: the two acoustic waves, the two vorticity waves (2D: the
+// entropy and the vorticity wave), and the two sides of the 3D entropy wave.
+__device__ __forceinline__ float2 f2(float x, float y) { return make_float2(x, y); }
+__device__ __forceinline__ float2 f2(float x) { return make_float2(x, x); }
+__device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
+__device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __ffma2_rn(b, f2(-1.f), a); }
+__device__ __forceinline__ float2 rcp2(float2 a) { return f2(rcp_approx(a.x), rcp_approx(a.y)); }
+__device__ __forceinline__ float2 abs2(float2 a) { return f2(fabsf(a.x), fabsf(a.y)); }
+
+// recon5 (FP32 form: see its epsilon) of two waves at once, on the differences of the stencil values.
+// s2: the square of the waves' scale (ReconEps), which the absolute epsilon of WENO5-JS takes.
+template <int SCH>
+__device__ __forceinline__ float2 recon5_x2(float2 fm2, float2 fm1, float2 f0, float2 fp1, float2 fp2, float eps_rel,
+                                            float ct, float2 s2) {
+  const float2 d1 = sub2(fm1, fm2), d2 = sub2(f0, fm1), d3 = sub2(fp1, f0), d4 = sub2(fp2, fp1);
+  const float2 c0 = sub2(d4, d3), s0 = fma2(f2(-2.f), d3, c0);  // [0, 1, 2]
+  const float2 c1 = sub2(d3, d2), s1 = add2(d2, d3);            // [-1, 0, 1]
+  const float2 c2 = sub2(d2, d1), s2_ = fma2(f2(2.f), d2, c2);  // [-2, -1, 0]
+  // four times epsilon: relative to the stencil's mean square, or WENO5-JS's constant
+  float2 e4;
+  if (SCH == SCH_WENO5_JS) {
+    e4 = mul2(f2(4.0e-6f), s2);
+  } else {
+    const float2 ss = fma2(fp2, fp2, fma2(fp1, fp1, fma2(f0, f0, fma2(fm1, fm1, mul2(fm2, fm2)))));
+    e4 = fma2(f2(0.8f * eps_rel), ss, f2(4e-30f));
+  }
+  const float2 k = f2((float)(13.0 / 3.0));
+  const float2 u0 = fma2(mul2(k, c0), c0, fma2(s0, s0, e4));
+  const float2 u1 = fma2(mul2(k, c1), c1, fma2(s1, s1, e4));
+  const float2 u2 = fma2(mul2(k, c2), c2, fma2(s2_, s2_, e4));
+  if (SCH == SCH_TENO5) {
+    const float2 tau = abs2(sub2(u1, u2));
+    float2 x0 = fma2(tau, rcp2(u0), f2(1.f)), x1 = fma2(tau, rcp2(u1), f2(1.f)), x2 = fma2(tau, rcp2(u2), f2(1.f));
+    const float2 im = f2(rcp_approx(fmaxf(x0.x, fmaxf(x1.x, x2.x))), rcp_approx(fmaxf(x0.y, fmaxf(x1.y, x2.y))));
+    x0 = mul2(x0, im);
+    x1 = mul2(x1, im);
+    x2 = mul2(x2, im);
+    x0 = mul2(mul2(x0, x0), x0); x0 = mul2(x0, x0);
+    x1 = mul2(mul2(x1, x1), x1); x1 = mul2(x1, x1);
+    x2 = mul2(mul2(x2, x2), x2); x2 = mul2(x2, x2);
+    const float2 cs = mul2(f2(ct), add2(add2(x0, x1), x2));
+    const float2 m0 = f2(x0.x < cs.x ? 0.f : 1.f, x0.y < cs.y ? 0.f : 1.f);
+    const float2 m1 = f2(x1.x < cs.x ? 0.f : 1.f, x1.y < cs.y ? 0.f : 1.f);
+    const float2 m2 = f2(x2.x < cs.x ? 0.f : 1.f, x2.y < cs.y ? 0.f : 1.f);
+    // weights times (e_r - f0): e0 - f0 = (4 d3 - d4) / 6, e1 - f0 = (d2 + 2 d3) / 6, e2 - f0 = (5 d2 - 2 d1) / 6
+    const float2 g0 = fma2(f2((float)(0.4 * 4.0 / 6.0)), d3, mul2(f2((float)(-0.4 / 6.0)), d4));
+    const float2 g1 = fma2(f2((float)(0.55 / 3.0)), d3, mul2(f2((float)(0.55 / 6.0)), d2));
+    const float2 g2 = fma2(f2((float)(0.05 * 5.0 / 6.0)), d2, mul2(f2((float)(-0.05 / 3.0)), d1));
+    const float2 Dn = fma2(f2(0.4f), m0, fma2(f2(0.55f), m1, mul2(f2(0.05f), m2)));
+    return fma2(fma2(m0, g0, fma2(m1, g1, mul2(m2, g2))), rcp2(Dn), f0);
+  }
+  float2 a0, a1, a2;  // the weights without the factors 3/10, 6/10, 1/10
+  if (SCH == SCH_WENO5_Z) {
+    const float2 tau = sub2(u0, u2);  // squared below
+    const float2 r0 = mul2(tau, rcp2(u0)), r1 = mul2(tau, rcp2(u1)), r2 = mul2(tau, rcp2(u2));
+    a0 = fma2(r0, r0, f2(1.f));
+    a1 = fma2(r1, r1, f2(1.f));
+    a2 = fma2(r2, r2, f2(1.f));
+  } else {
+    const float2 r0 = rcp2(u0), r1 = rcp2(u1), r2 = rcp2(u2);
+    const float2 im = f2(rcp_approx(fmaxf(r0.x, fmaxf(r1.x, r2.x))), rcp_approx(fmaxf(r0.y, fmaxf(r1.y, r2.y))));
+    a0 = mul2(r0, im); a0 = mul2(a0, a0);
+    a1 = mul2(r1, im); a1 = mul2(a1, a1);
+    a2 = mul2(r2, im); a2 = mul2(a2, a2);
+  }
+  // ten times the weights times (e_r - f0)
+  const float2 g0 = fma2(f2(2.f), d3, mul2(f2(-0.5f), d4));
+  const float2 g1 = fma2(f2(2.f), d3, d2);
+  const float2 g2 = fma2(f2((float)(5.0 / 6.0)), d2, mul2(f2((float)(-1.0 / 3.0)), d1));
+  const float2 Dn = fma2(f2(6.f), a1, fma2(f2(3.f), a0, a2));
+  return fma2(fma2(a0, g0, fma2(a1, g1, mul2(a2, g2))), rcp2(Dn), f0);
+}
+
+// FP32 characteristic LLF flux of a 2D / 3D interface in the factored form of char_flux_f64 (waves
+// scaled by a constant factor, projected flux in closed form) on packed pairs of waves.
+template <int ND, int SCH, int AVG>
+__device__ __forceinline__ void char_flux_f32(const Pt<float, ND> (&w)[6], const SP<float>& sp, float (&fh)[ND + 2]) {
+  constexpr int NV = ND + 2, E = ND + 1;
+  const float g1 = sp.g1;
+  const Pt<float, ND>& L = w[2];
+  const Pt<float, ND>& R = w[3];
+  float u[ND], a, ia, rho2, ke = 0.f;
+  if (AVG == AVG_ROE) {
+    const float iL = rsqrtf(L.q[0]), iR = rsqrtf(R.q[0]), sL = L.q[0] * iL, sR = R.q[0] * iR;
+    const float inv = rcp_approx(sL + sR), wl = sL * inv, wr = sR * inv;
+#pragma unroll
+    for (int i = 0; i < ND; ++i) {
+      u[i] = wl * L.u[i] + wr * R.u[i];
+      ke += u[i] * u[i];
+    }
+    const float H = ((L.q[E] + L.p) * iL + (R.q[E] + R.p) * iR) * inv;
+    const float a2 = g1 * (H - 0.5f * ke);
+    a = a2 * rsqrtf(a2);
+    rho2 = L.q[0] * R.q[0];
+  } else {
+#pragma unroll
+    for (int i = 0; i < ND; ++i) {
+      u[i] = 0.5f * (L.u[i] + R.u[i]);
+      ke += u[i] * u[i];
+    }
+    a = 0.5f * (L.a + R.a);
+    const float rho = 0.5f * (L.q[0] + R.q[0]);
+    rho2 = rho * rho;
+  }
+  ia = rcp_approx(a);
+  const float hk = 0.5f * ke, gi = g1 * ia, g = gi * ia;
+  const float lam_u = sp.sfc * fmaxf(fabsf(L.u[0]), fabsf(R.u[0]));
+  const float lam_p = sp.sfc * fmaxf(fabsf(L.u[0] + L.a), fabsf(R.u[0] + R.a));
+  const float lam_m = sp.sfc * fmaxf(fabsf(L.u[0] - L.a), fabsf(R.u[0] - R.a));
+  float P[6], W[6], up[6], um[6];
+#pragma unroll
+  for (int m = 0; m < 6; ++m) {
+    float x = w[m].q[E];
+#pragma unroll
+    for (int i = 0; i < ND; ++i) x = __fmaf_rn(-u[i], w[m].q[1 + i], x);
+    P[m] = __fmaf_rn(hk, w[m].q[0], x);
+    W[m] = w[m].p * (w[m].u[0] - u[0]);
+    up[m] = w[m].u[0] + lam_u;
+    um[m] = w[m].u[0] - lam_u;
+  }
+  auto sides = [&](const float2 (&fp)[6], const float2 (&fm)[6], float2 s2) -> float2 {
+    return add2(recon5_x2<SCH>(fp[0], fp[1], fp[2], fp[3], fp[4], sp.eps32_rel, sp.teno_ct, s2),
+                recon5_x2<SCH>(fm[5], fm[4], fm[3], fm[2], fm[1], sp.eps32_rel, sp.teno_ct, s2));
+  };
+  float2 fp[6], fm[6];
+  float r0, t1 = 0.f, t2;
+  if constexpr (ND == 3) {
+    // entropy wave: its + side and its mirrored - side are the pair
+    float p[6], q[6];
+#pragma unroll
+    for (int m = 0; m < 6; ++m) {
+      const float c = __fmaf_rn(-g, P[m], w[m].q[0]), t = g * W[m];
+      p[m] = __fmaf_rn(up[m], c, -t);
+      q[m] = __fmaf_rn(um[m], c, -t);
+    }
+    const float2 r = recon5_x2<SCH>(f2(p[0], q[5]), f2(p[1], q[4]), f2(p[2], q[3]), f2(p[3], q[2]), f2(p[4], q[1]),
+                                    sp.eps32_rel, sp.teno_ct, f2(4.f));
+    r0 = 0.5f * (r.x + r.y);
+    const float2 cu = f2(-u[ND - 1], u[1]);
+#pragma unroll
+    for (int m = 0; m < 6; ++m) {
+      const float2 c = fma2(cu, f2(w[m].q[0]), f2(w[m].q[ND], -w[m].q[2]));
+      fp[m] = mul2(f2(up[m]), c);
+      fm[m] = mul2(f2(um[m]), c);
+    }
+    const float2 v = sides(fp, fm, f2(4.f * rho2));
+    t1 = 0.5f * v.x;
+    t2 = 0.5f * v.y;
+  } else {
+    const float2 cu = f2(-g, u[1]);
+#pragma unroll
+    for (int m = 0; m < 6; ++m) {
+      const float2 c = fma2(cu, f2(P[m], w[m].q[0]), f2(w[m].q[0], -w[m].q[2]));
+      const float2 t = f2(-g * W[m], 0.f);
+      fp[m] = fma2(f2(up[m]), c, t);
+      fm[m] = fma2(f2(um[m]), c, t);
+    }
+    const float2 v = sides(fp, fm, f2(4.f, 4.f * rho2));
+    r0 = 0.5f * v.x;
+    t2 = 0.5f * v.y;
+  }
+  // acoustic waves u + a, u - a
+  const float2 lp = f2(lam_p, lam_m), lm = f2(-lam_p, -lam_m);
+#pragma unroll
+  for (int m = 0; m < 6; ++m) {
+    const float D = __fmaf_rn(-u[0], w[m].q[0], w[m].q[1]);
+    const float2 c = f2(__fmaf_rn(gi, P[m], D), __fmaf_rn(gi, P[m], -D));
+    const float2 f = fma2(f2(w[m].u[0]), c, f2(__fmaf_rn(gi, W[m], w[m].p), __fmaf_rn(gi, W[m], -w[m].p)));
+    fp[m] = fma2(lp, c, f);
+    fm[m] = fma2(lm, c, f);
+  }
+  const float2 r = sides(fp, fm, f2(8.f * rho2));
+  const float S = 0.25f * (r.x + r.y), B = 0.25f * (r.x - r.y), F0 = __fmaf_rn(ia, S, r0);
+  fh[0] = F0;
+  fh[1] = __fmaf_rn(u[0], F0, B);
+  fh[2] = __fmaf_rn(u[1], F0, -t2);
+  float e = __fmaf_rn(hk, F0, __fmaf_rn(a * sp.ig1, S, u[0] * B));
+  e = __fmaf_rn(-u[1], t2, e);
+  if constexpr (ND == 3) {
+    fh[ND] = __fmaf_rn(u[ND - 1], F0, t1);
+    e = __fmaf_rn(u[ND - 1], t1, e);
+  }
+  fh[NV - 1] = e;
+}
+
 // Characteristic LLF flux at the interface between w[2] and w[3] of a 6-point window
 // (offsets -2..+3), local frame.  Restates shock_capturing.py:786-891 and 979-1028 with the
 // eigensystems of euler_eigensystem.py for k = e_0.
@@ -616,6 +809,9 @@ template <typename T, int ND, int SCH, int AVG>
 __device__ __forceinline__ void char_flux(const Pt<T, ND> (&w)[6], const SP<T>& sp, T (&fh)[ND + 2]) {
   if constexpr (sizeof(T) == 8) {
     char_flux_f64<ND, SCH, AVG>(w, sp, fh);
+    return;
+  } else if constexpr (ND >= 2 && SCH != SCH_TENO6) {
+    char_flux_f32<ND, SCH, AVG>(w, sp, fh);
     return;
   }
   constexpr int NV = ND + 2;

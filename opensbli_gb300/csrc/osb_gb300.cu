@@ -592,14 +592,29 @@ __global__ void k_metric_f32(const double* m, float* out, long n) {
 
 // ---------------------------------------------------------------------------------------
 // Reductions (compressible_TGV.py:176-206 and the CFL / NaN checks), FP64.
-__device__ __forceinline__ double uval(const BlockK& b, int v, long id) { return b.q[v][id] / b.q[0][id]; }
-
-// d u_v / dx_d at the point (row j); a stretched y grid scales the y derivative by D11 of the row
-__device__ __forceinline__ double d1g(const BlockK& b, int v, long id, int d, int j) {
-  long s = b.st[d];
-  const double inv = (d == 1 && b.ys[0]) ? b.invd[1] * b.ys[0][j] : b.invd[d];
-  return ((1.0 / 12.0) * uval(b, v, id - 2 * s) - (2.0 / 3.0) * uval(b, v, id - s) + (2.0 / 3.0) * uval(b, v, id + s) -
-          (1.0 / 12.0) * uval(b, v, id + 2 * s)) * inv;
+// d u_v / dx_e at the point (row j) for the components v of mask[e], in g[v][e]; a stretched y grid
+// scales the y derivative by D11 of the row.  The reciprocal of a neighbour's density serves all of
+// its components: a point takes 12 of them instead of up to 24 divisions, which bounded the
+// enstrophy (FP64 pipe).
+__device__ __forceinline__ void vel_grad(const BlockK& b, long id, int j, const int (&mask)[3], double (&g)[3][3]) {
+  const double w[4] = {1.0 / 12.0, -2.0 / 3.0, 2.0 / 3.0, -1.0 / 12.0};
+  const int off[4] = {-2, -1, 1, 2};
+#pragma unroll
+  for (int e = 0; e < 3; ++e) {
+    if (e >= b.ndim) continue;
+    const double inv = (e == 1 && b.ys[0]) ? b.invd[1] * b.ys[0][j] : b.invd[e];
+    double s[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+      const long p = id + (long)off[m] * b.st[e];
+      const double ir = 1.0 / b.q[0][p];
+#pragma unroll
+      for (int v = 0; v < 3; ++v)
+        if (mask[e] >> v & 1) s[v] += w[m] * (b.q[1 + v][p] * ir);
+    }
+#pragma unroll
+    for (int v = 0; v < 3; ++v) g[v][e] = s[v] * inv;
+  }
 }
 
 struct RedParams {
@@ -632,22 +647,19 @@ __global__ void k_reduce(BlockK b, RedParams rp, double* partial, int slot) {
     switch (rp.what) {
       case 0: c = 0.5 * ke * rho; break;
       case 1: {
-        double w2 = 0.0;
-        if (nd == 3) {
-          double wx = d1g(b, 3, id, 1, j) - d1g(b, 2, id, 2, j);
-          double wy = d1g(b, 1, id, 2, j) - d1g(b, 3, id, 0, j);
-          double wz = d1g(b, 2, id, 0, j) - d1g(b, 1, id, 1, j);
-          w2 = wx * wx + wy * wy + wz * wz;
-        } else if (nd == 2) {
-          double wz = d1g(b, 2, id, 0, j) - d1g(b, 1, id, 1, j);
-          w2 = wz * wz;
-        }
-        c = w2 * mu;
+        const int mask[3] = {nd == 3 ? 6 : 2, nd == 3 ? 5 : 1, 3};
+        double g[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
+        vel_grad(b, id, j, mask, g);
+        const double wx = g[2][1] - g[1][2], wy = g[0][2] - g[2][0], wz = g[1][0] - g[0][1];
+        c = (nd == 3 ? wx * wx + wy * wy + wz * wz : nd == 2 ? wz * wz : 0.0) * mu;
         break;
       }
       case 2: {
+        const int mask[3] = {1, 2, 4};
+        double g[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
+        vel_grad(b, id, j, mask, g);
         double div = 0.0;
-        for (int e = 0; e < nd; ++e) div += d1g(b, 1 + e, id, e, j);
+        for (int e = 0; e < nd; ++e) div += g[e][e];
         c = (4.0 / 3.0) * div * div * mu;
         break;
       }
@@ -1885,17 +1897,20 @@ int osb_reduce(osb_ctx* c, int what, double* host_out) {
   const int threads = 256;
   for (auto& bl : c->blocks) {
     long n = (long)bl.k.n[0] * bl.k.n[1] * bl.k.n[2];
-    int grid = std::min(grid_for(c, n, threads), 64);
+    // one point per thread where the partials have room for it (up to 8 CTAs per SM; 64 CTAs, as few
+    // as each block had before, took 150 us of FP64 work for the enstrophy of a 64^3 block)
+    const long room = ((long)(c->red_slots + 8) * 64 - 1) / (long)c->blocks.size();
+    const int grid = std::min((long)grid_for(c, n, threads), std::max(64L, room));
     if (slot + grid > (c->red_slots + 8) * 64 - 1) return fail(OSB_ENOTSUP, "too many blocks for the reduction");
     RedParams rp{what, bl.d.ndim + 2, bl.d.viscous, bl.d.gama, bl.d.Minf, bl.d.mu_const, bl.d.visc_power};
     k_reduce<<<grid, threads, 0, c->stream>>>(bl.k, rp, c->red, slot);
     c->launches++;
     slot += grid;
   }
-  double* dout = c->red + ((size_t)(c->red_slots + 8) * 64 - 1);
-  k_reduce_final<<<1, 256, 0, c->stream>>>(c->red, slot, what == OSB_RED_CFL_DT, dout);
+  // the result goes straight to the pinned host word (device-accessible under unified addressing)
+  k_reduce_final<<<1, 256, 0, c->stream>>>(c->red, slot, what == OSB_RED_CFL_DT, c->red_host);
   c->launches++;
-  OSB_CK(cudaMemcpyAsync(c->red_host, dout, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+  OSB_CK(cudaGetLastError());
   OSB_CK(cudaStreamSynchronize(c->stream));
   *host_out = c->red_host[0];
   return OSB_OK;

@@ -2,19 +2,27 @@
 // path).
 //
 // One launch advances every block of the context by one RK stage.  The grid is persistent
-// (ctas_per_sm x SMs CTAs); each CTA claims 32 x ty point tiles of any block from a work list
-// (statically strided or through an atomic counter) and, per tile,
-//   1. stages the FP32 state of the tile plus 3 points on every side in shared memory, reading
+// (ctas_per_sm x SMs CTAs); each CTA claims tiles of up to 32 x ty points of any block from a work
+// list (one tile per CTA where they suffice, else statically strided or through an atomic counter)
+// and, per tile,
+//   1. stages the FP32 state of the tile plus 3 points on every side in shared memory with the
+//      primitives of each point (formed once), reading
 //      the periodic images directly from the opposite interior (equivalent to the periodic
 //      halo exchange of periodic.py:53-71, so no boundary kernel runs between stages),
-//   2. computes the characteristic LLF fluxes of the 33 x-interfaces of every row and the
-//      ty + 1 y-interfaces of every column into shared memory (char_flux, each flux once),
+//   2. computes the characteristic LLF fluxes of every x- and y-interface of the tile into shared
+//      memory, one interface per thread and round, both directions in one list (char_flux, each
+//      flux once),
 //   3. forms -(dF_x/dx + dF_y/dy) per point as a float-float pair (exact flux differences),
 //      applies the FP64 low-storage / SBLI RK update to the caller's state and register (the
 //      first low-storage stage, A = 0, does not read the register), and
 //      writes the FP32 state of the next stage into the other buffer of a ping-pong pair.
 // The residual never goes to HBM.  Tiles read one FP32 buffer and write the other, so a stage
 // has no intra-launch dependencies and needs no grid-wide barrier.
+//
+// Bound by the latency of the flux arithmetic at few warps: with a sliding window per thread a tile
+// gave each of its 128 threads nine interfaces in a row on 8 warps per SM (issue 40 %).  One interface
+// per thread and round needs 112 registers: 288 threads, 18 warps per SM with the default two CTAs,
+// four rounds for the 1 072 interfaces of a 32 x 16 tile.
 //
 // The tiling / schedule knobs (ty, CTAs per SM, static or dynamic claiming, work order) are
 // the analogue of OPS's cache-blocking tiling parameters (OPS_TILING, OPS_TILESIZE_X/Y) and are
@@ -28,9 +36,11 @@
 
 namespace osb {
 
-constexpr int BTX = 32;        // tile width (points)
-constexpr int BTHREADS = 128;  // threads per CTA
+constexpr int BTX = 32;        // largest tile width (points)
+constexpr int BTHREADS = 288;  // threads per CTA
 constexpr int BH = 3;          // stencil reach of the flux difference
+constexpr int BPITCH = BTX + 2 * BH;
+constexpr int BNF = 8;         // staged fields: rho, m0, m1, E, u0, u1, p, a
 
 struct BatchBlock {
   int n0, n1;       // interior size
@@ -42,20 +52,23 @@ struct BatchBlock {
   float* qout[4];
 };
 
-__device__ __forceinline__ int wrapi(int x, int n) { return x < 0 ? x + n : (x >= n ? x - n : x); }
+// Periodic image of x in [0, n) for x >= -n.
+__device__ __forceinline__ int wrapi(int x, int n) { return x < 0 ? x + n : (x < n ? x : x % n); }
+
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
 template <int SCH, int AVG>
-__global__ void __launch_bounds__(BTHREADS) k_batch2d(const BatchBlock* __restrict__ blocks,
+__global__ void __launch_bounds__(BTHREADS, 2) k_batch2d(const BatchBlock* __restrict__ blocks,
                                                       const int4* __restrict__ work, int nwork, int* counter,
                                                       int ty, SchemeParams spd, int kind, double A, double B,
                                                       float dt_h, float dt_l, int save, unsigned long long* bad) {
   constexpr int NV = 4;
   const SP<float> sp(spd);
   extern __shared__ __align__(16) unsigned char osb_smem[];
-  const int SP_ = BTX + 2 * BH;  // state pitch (38)
   const int SR = ty + 2 * BH;    // state rows
-  float* S = reinterpret_cast<float*>(osb_smem);  // [NV][SR][SP_]
-  float* Fx = S + NV * SR * SP_;                  // [NV][ty][BTX + 1]
+  const int SPL = SR * BPITCH;   // one staged field
+  float* S = reinterpret_cast<float*>(osb_smem);  // [BNF][SR][BPITCH]
+  float* Fx = S + BNF * SPL;                      // [NV][ty][BTX + 1]
   float* Fy = Fx + NV * ty * (BTX + 1);           // [NV][ty + 1][BTX]
   __shared__ int s_w;
   const int t = threadIdx.x;
@@ -75,80 +88,69 @@ __global__ void __launch_bounds__(BTHREADS) k_batch2d(const BatchBlock* __restri
     const BatchBlock& bk = blocks[wk.x];
     const int x0 = wk.y, y0 = wk.z;
     const int n0 = bk.n0, n1 = bk.n1;
-    // 1. stage the tile (periodic images read from the interior)
-    for (int idx = t; idx < NV * SR * SP_; idx += BTHREADS) {
-      const int c = idx % SP_, r = (idx / SP_) % SR, v = idx / (SP_ * SR);
-      const int gx = wrapi(x0 - BH + c, n0), gy = wrapi(y0 - BH + r, n1);
-      S[idx] = __ldg(bk.qin[v] + bk.off0 + gx + gy * bk.st1);
+    const int tw = min(wk.w & 0xffff, n0 - x0), th = min(wk.w >> 16, n1 - y0);  // the tile's points
+    // 1. stage the tile (periodic images read from the interior); the FP64 rows of phase 3 start
+    // towards L2 meanwhile
+    for (int idx = t; idx < (th + 2 * BH) * BPITCH; idx += BTHREADS) {
+      const int c = idx % BPITCH, r = idx / BPITCH;
+      if (c >= tw + 2 * BH) continue;
+      const int id = bk.off0 + wrapi(x0 - BH + c, n0) + wrapi(y0 - BH + r, n1) * bk.st1;
+      Pt<float, 2> s;
+#pragma unroll
+      for (int v = 0; v < NV; ++v) s.q[v] = __ldg(bk.qin[v] + id);
+      make_pt<float, 2>(s, gm);
+      float* at = S + idx;
+#pragma unroll
+      for (int v = 0; v < NV; ++v) at[v * SPL] = s.q[v];
+      at[4 * SPL] = s.u[0];
+      at[5 * SPL] = s.u[1];
+      at[6 * SPL] = s.p;
+      at[7 * SPL] = s.a;
+    }
+    for (int idx = t; idx < th * 2 * NV * 3; idx += BTHREADS) {
+      const int k = idx % 3, v = (idx / 3) % (2 * NV), r = idx / (6 * NV);
+      if (k * 16 < tw) prefetch_l2((v < NV ? bk.q[v] : bk.rk[v - NV]) + bk.off0 + x0 + k * 16 + (y0 + r) * bk.st1);
     }
     __syncthreads();
-    // 2a. x-interfaces i + 1/2, i = -1 .. 31, of each row: thread = (row, segment)
-    {
-      const int nseg = BTHREADS / ty;
-      const int per = (BTX + 1 + nseg - 1) / nseg;
-      const int row = t % ty, seg = t / ty;
-      const int i0 = -1 + seg * per, i1 = min(BTX, i0 + per);
-      const float* Sr = S + (row + BH) * SP_;
+    // 2. x-interfaces i = 0 .. tw of each row (left of point i), then y-interfaces j = 0 .. th of
+    // each column; the local frame of y has u1 as the normal velocity
+    const int nx = (tw + 1) * th, nall = nx + tw * (th + 1);
+    for (int k = t; k < nall; k += BTHREADS) {
+      const bool yd = k >= nx;
+      const int kk = yd ? k - nx : k, wd = yd ? tw : tw + 1;
+      const int r = kk / wd, c = kk - r * wd;
+      // first point of the window: three left of (below) the interface's right (upper) point
+      const float* s = S + (yd ? r * BPITCH + c + BH : (r + BH) * BPITCH + c);
+      const int st = yd ? BPITCH : 1;
+      const int fn = yd ? 2 : 1, ft = 3 - fn;
       Pt<float, 2> win[6];
-      if (i0 < i1) {
 #pragma unroll
-        for (int m = 1; m < 6; ++m) {
-          const int col = i0 + m - 3 + BH;  // point i0 - 3 + m
-#pragma unroll
-          for (int v = 0; v < NV; ++v) win[m].q[v] = Sr[v * SR * SP_ + col];
-          make_pt<float, 2>(win[m], gm);
-        }
+      for (int m = 0; m < 6; ++m) {
+        const float* a = s + m * st;
+        win[m].q[0] = a[0];
+        win[m].q[1] = a[fn * SPL];
+        win[m].q[2] = a[ft * SPL];
+        win[m].q[3] = a[3 * SPL];
+        win[m].u[0] = a[(3 + fn) * SPL];
+        win[m].u[1] = a[(3 + ft) * SPL];
+        win[m].p = a[6 * SPL];
+        win[m].a = a[7 * SPL];
       }
-      for (int i = i0; i < i1; ++i) {
-#pragma unroll
-        for (int m = 0; m < 5; ++m) win[m] = win[m + 1];
-        const int col = i + 3 + BH;
-#pragma unroll
-        for (int v = 0; v < NV; ++v) win[5].q[v] = Sr[v * SR * SP_ + col];
-        make_pt<float, 2>(win[5], gm);
-        float fh[NV];
-        char_flux<float, 2, SCH, AVG>(win, sp, fh);
-#pragma unroll
-        for (int v = 0; v < NV; ++v) Fx[(v * ty + row) * (BTX + 1) + i + 1] = fh[v];
-      }
-    }
-    // 2b. y-interfaces j + 1/2, j = -1 .. ty-1, of each column (local frame: normal = u1)
-    {
-      const int nseg = BTHREADS / BTX;
-      const int per = (ty + 1 + nseg - 1) / nseg;
-      const int col = t % BTX, seg = t / BTX;
-      const int j0 = -1 + seg * per, j1 = min(ty, j0 + per);
-      const float* Sc = S + col + BH;
-      Pt<float, 2> win[6];
-      if (j0 < j1) {
-#pragma unroll
-        for (int m = 1; m < 6; ++m) {
-          const int r = j0 + m - 3 + BH;
-#pragma unroll
-          for (int lv = 0; lv < NV; ++lv) win[m].q[lv] = Sc[gvar<2, 1, false>(lv) * SR * SP_ + r * SP_];
-          make_pt<float, 2>(win[m], gm);
-        }
-      }
-      for (int j = j0; j < j1; ++j) {
-#pragma unroll
-        for (int m = 0; m < 5; ++m) win[m] = win[m + 1];
-        const int r = j + 3 + BH;
-#pragma unroll
-        for (int lv = 0; lv < NV; ++lv) win[5].q[lv] = Sc[gvar<2, 1, false>(lv) * SR * SP_ + r * SP_];
-        make_pt<float, 2>(win[5], gm);
-        float fh[NV];
-        char_flux<float, 2, SCH, AVG>(win, sp, fh);
-#pragma unroll
-        for (int lv = 0; lv < NV; ++lv) Fy[(gvar<2, 1, false>(lv) * (ty + 1) + j + 1) * BTX + col] = fh[lv];
-      }
+      float fh[NV];
+      char_flux<float, 2, SCH, AVG>(win, sp, fh);
+      float* f = yd ? Fy + r * BTX + c : Fx + r * (BTX + 1) + c;
+      const int fs = yd ? (ty + 1) * BTX : ty * (BTX + 1);
+      f[0] = fh[0];
+      f[fn * fs] = fh[1];
+      f[ft * fs] = fh[2];
+      f[3 * fs] = fh[3];
     }
     __syncthreads();
     // 3. residual (float-float) and FP64 RK update of the tile's points
-    for (int p = t; p < BTX * ty; p += BTHREADS) {
+    for (int p = t; p < BTX * th; p += BTHREADS) {
       const int r = p / BTX, c = p % BTX;
-      const int gx = x0 + c, gy = y0 + r;
-      if (gx >= n0 || gy >= n1) continue;
-      const int id = bk.off0 + gx + gy * bk.st1;
+      if (c >= tw) continue;
+      const int id = bk.off0 + x0 + c + (y0 + r) * bk.st1;
 #pragma unroll
       for (int v = 0; v < NV; ++v) {
         float p1, e1, p2, e2;
@@ -181,8 +183,8 @@ __global__ void __launch_bounds__(BTHREADS) k_batch2d(const BatchBlock* __restri
 
 size_t batch_smem(int ty) {
   const int NV = 4;
-  return sizeof(float) * ((size_t)NV * (ty + 2 * BH) * (BTX + 2 * BH) + (size_t)NV * ty * (BTX + 1) +
-                          (size_t)NV * (ty + 1) * BTX);
+  return sizeof(float) *
+         ((size_t)BNF * (ty + 2 * BH) * BPITCH + (size_t)NV * ty * (BTX + 1) + (size_t)NV * (ty + 1) * BTX);
 }
 
 namespace {
@@ -192,15 +194,15 @@ int launch_batch_t(osb_ctx* c, const BatchBlock* tab, const SchemeParams& sp, in
                    int save) {
   const float dt_h = (float)dt, dt_l = (float)(dt - (double)dt_h);
   auto kern = k_batch2d<SCH, AVG>;
-  const int ty = c->sched.tile_y;
+  const int ty = c->batch.ty;
   const size_t smem = batch_smem(ty);
   OSB_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   int* counter = nullptr;
-  if (c->sched.dynamic) {
+  const int grid = std::max(1, std::min(c->batch.nwork, c->sched.ctas_per_sm * c->sm_count));
+  if (c->sched.dynamic && grid < c->batch.nwork) {  // a CTA per tile has nothing to claim
     OSB_CK(cudaMemsetAsync(c->batch.counter, 0, sizeof(int), c->stream));
     counter = c->batch.counter;
   }
-  const int grid = std::max(1, std::min(c->batch.nwork, c->sched.ctas_per_sm * c->sm_count));
   timing_begin(c, FAM_PERSISTENT);
   kern<<<grid, BTHREADS, smem, c->stream>>>(tab, c->batch.work, c->batch.nwork, counter, ty, sp, kind, A, B, dt_h,
                                             dt_l, save, c->bad);
@@ -235,9 +237,22 @@ bool batch_eligible(const osb_ctx* c, std::string* why) {
 // work list for the current schedule.
 int batch_build(osb_ctx* c) {
   batch_free(c);
-  const int ty = c->sched.tile_y;
-  if (ty != 8 && ty != 16 && ty != 32) return fail(OSB_EINVAL, "tile_y must be 8, 16 or 32");
+  if (c->sched.tile_y != 8 && c->sched.tile_y != 16 && c->sched.tile_y != 32)
+    return fail(OSB_EINVAL, "tile_y must be 8, 16 or 32");
   const int nb = (int)c->blocks.size();
+  // Tiles are at most 32 x tile_y points, a block's extents cut evenly.  Where tiles of that height
+  // do not give every SM one, lower ones do: the launch then lasts as long as one tile, and the
+  // extra y-interface per column of a lower tile costs less than the idle SMs (97 x 120 points: 32
+  // tiles of height 16 took 27 us a stage, see the header for the time now).
+  auto parts = [](int n, int most) { return (n + most - 1) / most; };
+  auto tiles = [&](int h) {
+    long n = 0;
+    for (const auto& bl : c->blocks) n += (long)parts(bl.k.n[0], BTX) * parts(bl.k.n[1], h);
+    return n;
+  };
+  int ty = c->sched.tile_y;
+  while (ty > 2 && tiles(ty) < c->sm_count) ty /= 2;
+  c->batch.ty = ty;
   std::vector<BatchBlock> tab[2];
   for (int ib = 0; ib < nb; ++ib) {
     Block& bl = c->blocks[ib];
@@ -270,8 +285,9 @@ int batch_build(osb_ctx* c) {
   std::vector<std::vector<int4>> per(nb);
   for (int ib = 0; ib < nb; ++ib) {
     const BlockK& k = c->blocks[ib].k;
-    for (int y = 0; y < k.n[1]; y += ty)
-      for (int x = 0; x < k.n[0]; x += BTX) per[ib].push_back(make_int4(ib, x, y, 0));
+    const int tw = parts(k.n[0], parts(k.n[0], BTX)), th = parts(k.n[1], parts(k.n[1], ty));
+    for (int y = 0; y < k.n[1]; y += th)
+      for (int x = 0; x < k.n[0]; x += tw) per[ib].push_back(make_int4(ib, x, y, tw | th << 16));
   }
   std::vector<int4> work;
   if (c->sched.order == 2) {

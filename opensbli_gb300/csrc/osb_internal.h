@@ -37,7 +37,8 @@ struct BatchBlock;
 // Device tables of the persistent stage (osb_batch.cu).
 struct BatchState {
   BatchBlock* tab[2] = {nullptr, nullptr};  // per FP32-buffer parity
-  int4* work = nullptr;                     // tiles: (block, x0, y0, -)
+  int4* work = nullptr;                     // tiles: (block, x0, y0, width | height << 16)
+  int ty = 0;                               // largest tile height of the list
   int* counter = nullptr;                   // dynamic tile claiming
   int nwork = 0;
   bool ready = false;

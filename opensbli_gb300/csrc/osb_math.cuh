@@ -443,6 +443,19 @@ __device__ __forceinline__ void make_pt(Pt<T, ND>& s, T gm) {
   s.a = sqrt(gm * s.p * ir);
 }
 
+// FP32 2D: the kinetic energy as a sum of two rounded squares, which does not depend on the order of
+// the components: the persistent stage forms a point's primitives once for both directions, the
+// sweeps in each direction's own frame, and they agree bit for bit.
+template <typename T, int ND>
+__device__ __forceinline__ void make_pt(Pt<float, 2>& s, float gm) {
+  const float ir = 1.0f / s.q[0];
+  s.u[0] = __fmul_rn(s.q[1], ir);
+  s.u[1] = __fmul_rn(s.q[2], ir);
+  const float ke = __fadd_rn(__fmul_rn(s.u[0], s.u[0]), __fmul_rn(s.u[1], s.u[1]));
+  s.p = __fmul_rn(gm - 1.0f, __fmaf_rn(__fmul_rn(-0.5f, s.q[0]), ke, s.q[3]));
+  s.a = sqrtf(__fmul_rn(__fmul_rn(gm, s.p), ir));
+}
+
 // FP64: the square root of the density and the total enthalpy that the Roe average takes from
 // either side of an interface are formed once per point (a point is a side of two interfaces).
 template <int ND>
@@ -691,7 +704,9 @@ __device__ __forceinline__ float2 recon5_x2(float2 fm2, float2 fm1, float2 f0, f
 }
 
 // FP32 characteristic LLF flux of a 2D / 3D interface in the factored form of char_flux_f64 (waves
-// scaled by a constant factor, projected flux in closed form) on packed pairs of waves.
+// scaled by a constant factor, projected flux in closed form) on packed pairs of waves.  Products
+// that feed sums are written as explicit multiply-adds: the sweeps and the persistent stage inline
+// this into different code and still give the same bits.
 template <int ND, int SCH, int AVG>
 __device__ __forceinline__ void char_flux_f32(const Pt<float, ND> (&w)[6], const SP<float>& sp, float (&fh)[ND + 2]) {
   constexpr int NV = ND + 2, E = ND + 1;
@@ -704,18 +719,18 @@ __device__ __forceinline__ void char_flux_f32(const Pt<float, ND> (&w)[6], const
     const float inv = rcp_approx(sL + sR), wl = sL * inv, wr = sR * inv;
 #pragma unroll
     for (int i = 0; i < ND; ++i) {
-      u[i] = wl * L.u[i] + wr * R.u[i];
-      ke += u[i] * u[i];
+      u[i] = __fmaf_rn(wl, L.u[i], __fmul_rn(wr, R.u[i]));
+      ke = __fmaf_rn(u[i], u[i], ke);
     }
-    const float H = ((L.q[E] + L.p) * iL + (R.q[E] + R.p) * iR) * inv;
-    const float a2 = g1 * (H - 0.5f * ke);
+    const float H = __fmul_rn(__fmaf_rn(L.q[E] + L.p, iL, __fmul_rn(R.q[E] + R.p, iR)), inv);
+    const float a2 = __fmul_rn(g1, __fmaf_rn(-0.5f, ke, H));
     a = a2 * rsqrtf(a2);
     rho2 = L.q[0] * R.q[0];
   } else {
 #pragma unroll
     for (int i = 0; i < ND; ++i) {
       u[i] = 0.5f * (L.u[i] + R.u[i]);
-      ke += u[i] * u[i];
+      ke = __fmaf_rn(u[i], u[i], ke);
     }
     a = 0.5f * (L.a + R.a);
     const float rho = 0.5f * (L.q[0] + R.q[0]);
@@ -733,7 +748,7 @@ __device__ __forceinline__ void char_flux_f32(const Pt<float, ND> (&w)[6], const
 #pragma unroll
     for (int i = 0; i < ND; ++i) x = __fmaf_rn(-u[i], w[m].q[1 + i], x);
     P[m] = __fmaf_rn(hk, w[m].q[0], x);
-    W[m] = w[m].p * (w[m].u[0] - u[0]);
+    W[m] = __fmul_rn(w[m].p, w[m].u[0] - u[0]);
     up[m] = w[m].u[0] + lam_u;
     um[m] = w[m].u[0] - lam_u;
   }
@@ -748,7 +763,7 @@ __device__ __forceinline__ void char_flux_f32(const Pt<float, ND> (&w)[6], const
     float p[6], q[6];
 #pragma unroll
     for (int m = 0; m < 6; ++m) {
-      const float c = __fmaf_rn(-g, P[m], w[m].q[0]), t = g * W[m];
+      const float c = __fmaf_rn(-g, P[m], w[m].q[0]), t = __fmul_rn(g, W[m]);
       p[m] = __fmaf_rn(up[m], c, -t);
       q[m] = __fmaf_rn(um[m], c, -t);
     }
@@ -770,7 +785,7 @@ __device__ __forceinline__ void char_flux_f32(const Pt<float, ND> (&w)[6], const
 #pragma unroll
     for (int m = 0; m < 6; ++m) {
       const float2 c = fma2(cu, f2(P[m], w[m].q[0]), f2(w[m].q[0], -w[m].q[2]));
-      const float2 t = f2(-g * W[m], 0.f);
+      const float2 t = f2(__fmul_rn(-g, W[m]), 0.f);
       fp[m] = fma2(f2(up[m]), c, t);
       fm[m] = fma2(f2(um[m]), c, t);
     }
@@ -789,11 +804,11 @@ __device__ __forceinline__ void char_flux_f32(const Pt<float, ND> (&w)[6], const
     fm[m] = fma2(lm, c, f);
   }
   const float2 r = sides(fp, fm, f2(8.f * rho2));
-  const float S = 0.25f * (r.x + r.y), B = 0.25f * (r.x - r.y), F0 = __fmaf_rn(ia, S, r0);
+  const float S = __fmul_rn(0.25f, r.x + r.y), B = __fmul_rn(0.25f, r.x - r.y), F0 = __fmaf_rn(ia, S, r0);
   fh[0] = F0;
   fh[1] = __fmaf_rn(u[0], F0, B);
   fh[2] = __fmaf_rn(u[1], F0, -t2);
-  float e = __fmaf_rn(hk, F0, __fmaf_rn(a * sp.ig1, S, u[0] * B));
+  float e = __fmaf_rn(hk, F0, __fmaf_rn(__fmul_rn(a, sp.ig1), S, __fmul_rn(u[0], B)));
   e = __fmaf_rn(-u[1], t2, e);
   if constexpr (ND == 3) {
     fh[ND] = __fmaf_rn(u[ND - 1], F0, t1);

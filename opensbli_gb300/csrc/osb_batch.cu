@@ -21,8 +21,9 @@
 //
 // Bound by the latency of the flux arithmetic at few warps: with a sliding window per thread a tile
 // gave each of its 128 threads nine interfaces in a row on 8 warps per SM (issue 40 %).  One interface
-// per thread and round needs 112 registers: 288 threads, 18 warps per SM with the default two CTAs,
-// four rounds for the 1 072 interfaces of a 32 x 16 tile.
+// per thread and round fits 80 registers: 384 threads, 24 warps per SM with the default two CTAs,
+// three rounds for the 1 072 interfaces of a 32 x 16 tile.  The phases between the rounds wait on
+// memory, so a tile's FP64 rows and the next tile's FP32 rows are prefetched into L2.
 //
 // The tiling / schedule knobs (ty, CTAs per SM, static or dynamic claiming, work order) are
 // the analogue of OPS's cache-blocking tiling parameters (OPS_TILING, OPS_TILESIZE_X/Y) and are
@@ -37,7 +38,7 @@
 namespace osb {
 
 constexpr int BTX = 32;        // largest tile width (points)
-constexpr int BTHREADS = 288;  // threads per CTA
+constexpr int BTHREADS = 384;  // threads per CTA
 constexpr int BH = 3;          // stencil reach of the flux difference
 constexpr int BPITCH = BTX + 2 * BH;
 constexpr int BNF = 8;         // staged fields: rho, m0, m1, E, u0, u1, p, a
@@ -45,6 +46,8 @@ constexpr int BNF = 8;         // staged fields: rho, m0, m1, E, u0, u1, p, a
 struct BatchBlock {
   int n0, n1;       // interior size
   int st1, off0;    // OPS-layout row stride and linear index of (0, 0)
+  int depth;        // exchange depth of its (periodic) faces, one for all; 0: they differ
+  long alloc;       // allocated points per array
   float invd0, invd1;
   double* q[4];
   double* rk[4];
@@ -74,16 +77,11 @@ __global__ void __launch_bounds__(BTHREADS, 2) k_batch2d(const BatchBlock* __res
   const int t = threadIdx.x;
   const float gm = sp.gama;
   unsigned long long nbad = 0;
-  for (int it = 0;; ++it) {
-    int w;
-    if (counter) {
-      if (t == 0) s_w = atomicAdd(counter, 1);
-      __syncthreads();
-      w = s_w;
-    } else {
-      w = blockIdx.x + it * gridDim.x;
-    }
-    if (w >= nwork) break;
+  // dynamic claiming takes the next tile while the current one is computed (the first one is the
+  // CTA's own number: the counter starts at the grid size)
+  int w = blockIdx.x;
+  while (w < nwork) {
+    if (counter && t == 0) s_w = atomicAdd(counter, 1) + gridDim.x;
     const int4 wk = work[w];
     const BatchBlock& bk = blocks[wk.x];
     const int x0 = wk.y, y0 = wk.z;
@@ -112,6 +110,17 @@ __global__ void __launch_bounds__(BTHREADS, 2) k_batch2d(const BatchBlock* __res
       if (k * 16 < tw) prefetch_l2((v < NV ? bk.q[v] : bk.rk[v - NV]) + bk.off0 + x0 + k * 16 + (y0 + r) * bk.st1);
     }
     __syncthreads();
+    w = counter ? s_w : w + gridDim.x;
+    if (w < nwork) {  // the next tile's FP32 rows towards L2
+      const int4 nk = work[w];
+      const BatchBlock& nb = blocks[nk.x];
+      const int nw = min(nk.w & 0xffff, nb.n0 - nk.y), nh = min(nk.w >> 16, nb.n1 - nk.z);
+      for (int idx = t; idx < (nh + 2 * BH) * NV * 2; idx += BTHREADS) {
+        const int k = idx & 1, v = (idx >> 1) % NV, r = idx / (2 * NV);
+        if (k == 0 || nw > 1)
+          prefetch_l2(nb.qin[v] + nb.off0 + nk.y + (k ? nw - 1 : 0) + wrapi(nk.z - BH + r, nb.n1) * nb.st1);
+      }
+    }
     // 2. x-interfaces i = 0 .. tw of each row (left of point i), then y-interfaces j = 0 .. th of
     // each column; the local frame of y has u1 as the normal velocity
     const int nx = (tw + 1) * th, nall = nx + tw * (th + 1);
@@ -179,6 +188,43 @@ __global__ void __launch_bounds__(BTHREADS, 2) k_batch2d(const BatchBlock* __res
     __syncthreads();  // the next tile reuses the shared arrays (and s_w)
   }
   if (nbad) atomicAdd(bad, nbad);
+}
+
+// FP32 state <- FP64 state of every block, whole allocations (k_q2qf of all blocks in one launch;
+// blockIdx.y = 4 * block + variable).
+__global__ void k_batch_q2qf(const BatchBlock* __restrict__ blocks) {
+  const BatchBlock& b = blocks[blockIdx.y >> 2];
+  const int v = blockIdx.y & 3, n = (int)b.alloc;
+  float* f = const_cast<float*>(b.qin[v]);
+  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) f[t] = d2f_rn(b.q[v][t]);
+}
+
+// Periodic halo shells of every block, FP64 and FP32 state (k_periodic_shell of all blocks in one
+// launch; blockIdx.y = block): y faces over the full row, then x faces of the interior rows.
+__global__ void k_batch_halo(const BatchBlock* __restrict__ blocks) {
+  const BatchBlock& b = blocks[blockIdx.y];
+  const int D = b.depth, n0 = b.n0, n1 = b.n1, e0 = n0 + 2 * D;
+  const int cy = 2 * D * e0, total = cy + 2 * D * n1;
+  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
+    int x, y;
+    if (t < cy) {
+      x = t % e0 - D;
+      y = t / e0;
+      y = y < D ? y - D : n1 + y - D;
+    } else {
+      const int u = t - cy;
+      x = u % (2 * D);
+      x = x < D ? x - D : n0 + x - D;
+      y = u / (2 * D);
+    }
+    const int di = b.off0 + x + y * b.st1, si = b.off0 + wrapi(x, n0) + wrapi(y, n1) * b.st1;
+#pragma unroll
+    for (int v = 0; v < 4; ++v) {
+      b.q[v][di] = b.q[v][si];
+      float* f = const_cast<float*>(b.qin[v]);
+      f[di] = f[si];
+    }
+  }
 }
 
 size_t batch_smem(int ty) {
@@ -265,6 +311,8 @@ int batch_build(osb_ctx* c) {
       b.n1 = bl.k.n[1];
       b.st1 = bl.k.st[1];
       b.off0 = bl.k.off0;
+      b.alloc = bl.k.alloc;
+      b.depth = bl.periodic_depth();
       b.invd0 = (float)bl.k.invd[0];
       b.invd1 = (float)bl.k.invd[1];
       for (int v = 0; v < 4; ++v) {
@@ -301,6 +349,12 @@ int batch_build(osb_ctx* c) {
     for (int ib : order) work.insert(work.end(), per[ib].begin(), per[ib].end());
   }
   c->batch.nwork = (int)work.size();
+  c->batch.one_depth = true;
+  c->batch.max_alloc = 0;
+  for (const auto& bl : c->blocks) {
+    c->batch.one_depth = c->batch.one_depth && bl.periodic_depth() > 0;
+    c->batch.max_alloc = std::max(c->batch.max_alloc, bl.k.alloc);
+  }
   for (int p = 0; p < 2; ++p) {
     OSB_CK(cudaMalloc(&c->batch.tab[p], sizeof(BatchBlock) * nb));
     OSB_CK(cudaMemcpyAsync(c->batch.tab[p], tab[p].data(), sizeof(BatchBlock) * nb, cudaMemcpyHostToDevice,
@@ -326,6 +380,25 @@ void batch_free(osb_ctx* c) {
   c->batch.counter = nullptr;
   c->batch.nwork = 0;
   c->batch.ready = false;
+}
+
+// The FP32 state of every block from its FP64 state, and the halos of both at the end of a call, each
+// in one launch (128 launches for 64 instances before, 0.9 ms of a 5-step call).  False where the
+// tables do not allow it: the caller then goes block by block.
+bool batch_sync_shadow(osb_ctx* c) {
+  if (!c->batch.ready || c->blocks.size() > 16383) return false;
+  const dim3 grid((unsigned)std::min(grid_for(c, c->batch.max_alloc, 256), 64), (unsigned)(4 * c->blocks.size()));
+  k_batch_q2qf<<<grid, 256, 0, c->stream>>>(c->batch.tab[c->qf_parity]);
+  c->launches++;
+  return true;
+}
+bool batch_halo(osb_ctx* c) {
+  if (!c->batch.ready || !c->batch.one_depth || c->blocks.size() > 65535) return false;
+  timing_begin(c, FAM_BC);
+  k_batch_halo<<<dim3(8, (unsigned)c->blocks.size()), 256, 0, c->stream>>>(c->batch.tab[c->qf_parity]);
+  timing_end(c);
+  c->launches++;
+  return true;
 }
 
 // Points BlockK::qf of every block at FP32 buffer `parity` (0: the original one).

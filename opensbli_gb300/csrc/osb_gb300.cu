@@ -209,22 +209,6 @@ __global__ void k_periodic_shell(BlockK b, int nv, int D, int fields) {
   }
 }
 
-// Depth of a block whose faces are all periodic with one depth D not above any of its
-// extents (so one wrap lands in the interior), else 0.
-static int uniform_periodic_depth(const Block& bl) {
-  int D = 0;
-  for (int d = 0; d < bl.d.ndim; ++d)
-    for (int side = 0; side < 2; ++side) {
-      if (bl.d.bc[d][side] != OSB_BC_PERIODIC) return 0;
-      const int dep = bl.d.bc_depth[d][side] > 0 ? bl.d.bc_depth[d][side] : 4;
-      if (D == 0) D = dep;
-      else if (dep != D) return 0;
-    }
-  for (int d = 0; d < bl.d.ndim; ++d)
-    if (bl.k.n[d] < D) return 0;
-  return D;
-}
-
 // Zero-gradient outlet (zero_gradient_outlet.py:11-23 as generated): on side 0,
 // q(0) = q(1) then q(-m) = q(m) for m = 1..depth; mirrored on side 1.  Over the interior
 // extent of the other directions.
@@ -910,7 +894,7 @@ bool block_faces_ok(const osb_block_desc& d, std::string& why) {
 // symmetry, Dirichlet, pressure-outlet and wall faces.
 int apply_block_bc(osb_ctx* c, Block& bl, size_t ib, int fields) {
   const int nv = bl.d.ndim + 2;
-  if (const int D = uniform_periodic_depth(bl)) {
+  if (const int D = bl.periodic_depth()) {
     long shell = 1, inner = 1;
     for (int e = 0; e < bl.d.ndim; ++e) {
       shell *= bl.k.n[e] + 2 * D;
@@ -1088,6 +1072,7 @@ bool any_filter(const osb_ctx* c, int kind) {
 // have written q between calls).
 int sync_shadow(osb_ctx* c) {
   if (c->prec != OSB_PREC_FP32_RESIDUAL) return OSB_OK;
+  if (use_batch(c) && batch_sync_shadow(c)) return OSB_OK;
   for (auto& bl : c->blocks) {
     dim3 grid(grid_for(c, bl.k.alloc, 256), bl.d.ndim + 2);
     k_q2qf<<<grid, 256, 0, c->stream>>>(bl.k, bl.d.ndim + 2);
@@ -1771,6 +1756,16 @@ int osb_apply_bc(osb_ctx* c) {
   return OSB_OK;
 }
 
+namespace {
+
+// Halos that a caller observes when a call of the FP32-residual path returns.
+int observer_halos(osb_ctx* c, bool batch) {
+  if (batch && batch_halo(c)) return OSB_OK;
+  return apply_bc(c, batch ? BC_BOTH : BC_Q);
+}
+
+}  // namespace
+
 int osb_step(osb_ctx* c, double dt, int nsteps) {
   if (!c) return fail(OSB_EINVAL, "null ctx");
   if (nsteps < 0) return fail(OSB_EINVAL, "nsteps < 0");
@@ -1784,20 +1779,20 @@ int osb_step(osb_ctx* c, double dt, int nsteps) {
     OSB_CK(cudaGetLastError());
     return OSB_OK;
   }
-  int src = sync_shadow(c);
-  if (src) return src;
   const bool batch = use_batch(c);
   if (batch && !c->batch.ready) {
     int rc = batch_build(c);  // allocates: never inside a capture
     if (rc) return rc;
   }
+  int src = sync_shadow(c);
+  if (src) return src;
   if (!c->graphs || c->timing) {
     for (int it = 0; it < nsteps; ++it) {
       int rc = one_step(c, dt);
       if (rc) return rc;
     }
     if (c->prec == OSB_PREC_FP32_RESIDUAL) {
-      int rc = apply_bc(c, batch ? BC_BOTH : BC_Q);  // halos for observers
+      int rc = observer_halos(c, batch);
       if (rc) return rc;
     }
     OSB_CK(cudaGetLastError());
@@ -1834,7 +1829,7 @@ int osb_step(osb_ctx* c, double dt, int nsteps) {
       batch_set_parity(c, p ^ (c->nst & 1));
     }
     {
-      int rc = apply_bc(c, batch ? BC_BOTH : BC_Q);  // halos of the FP64 (and FP32) state for observers
+      int rc = observer_halos(c, batch);
       if (rc) return rc;
     }
     OSB_CK(cudaGetLastError());

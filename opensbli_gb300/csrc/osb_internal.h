@@ -26,6 +26,21 @@ struct Block {
   float* qf_base = nullptr;  // FP32 state buffer allocated with the block (FP32-residual path)
   float* qf_alt = nullptr;   // second FP32 state buffer of the persistent stage's ping-pong
   void* filt_ws = nullptr;   // filtered blocks: kappa + 15 filter-flux arrays (residual precision)
+  // Depth of a block whose faces are all periodic with one depth D not above any of its
+  // extents (so one wrap lands in the interior), else 0.
+  int periodic_depth() const {
+    int D = 0;
+    for (int e = 0; e < d.ndim; ++e)
+      for (int side = 0; side < 2; ++side) {
+        if (d.bc[e][side] != OSB_BC_PERIODIC) return 0;
+        const int dep = d.bc_depth[e][side] > 0 ? d.bc_depth[e][side] : 4;
+        if (D == 0) D = dep;
+        else if (dep != D) return 0;
+      }
+    for (int e = 0; e < d.ndim; ++e)
+      if (k.n[e] < D) return 0;
+    return D;
+  }
   int* xrows = nullptr;      // x-sweep rows (linear index of x = 0) grouped by 32-byte-sector phase
 };
 
@@ -39,6 +54,8 @@ struct BatchState {
   BatchBlock* tab[2] = {nullptr, nullptr};  // per FP32-buffer parity
   int4* work = nullptr;                     // tiles: (block, x0, y0, width | height << 16)
   int ty = 0;                               // largest tile height of the list
+  bool one_depth = false;                   // every block's faces have one exchange depth
+  long max_alloc = 0;                       // allocated points of the largest block
   int* counter = nullptr;                   // dynamic tile claiming
   int nwork = 0;
   bool ready = false;
@@ -118,6 +135,8 @@ int batch_build(osb_ctx* c);
 void batch_free(osb_ctx* c);
 void batch_set_parity(osb_ctx* c, int parity);
 int batch_stage(osb_ctx* c, int s, double dt);
+bool batch_sync_shadow(osb_ctx* c);
+bool batch_halo(osb_ctx* c);
 size_t batch_smem(int ty);
 // Central convective and/or viscous terms of one 3D block (osb_central.cu).
 // Resident CTAs per SM of a kernel at a launch shape (occupancy calculator; 1 if it fails).

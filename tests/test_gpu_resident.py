@@ -94,3 +94,31 @@ def test_resident_1d_fp32_residual(built_lib, oracle_lib, bc):
     for v in range(spec.nvars):
         assert harness.rel_err(res[v][sl], per[v][sl]) < 1e-5, (bc, v, "per-block")
         assert harness.rel_err(res[v][sl], ob.q[0][v][sl]) < 1e-4, (bc, v, "oracle")
+
+
+@pytest.mark.parametrize("bc", sorted(BCS))
+@pytest.mark.parametrize("sizes", [(6,), (11, 12), (31,), (32, 33), (62, 63), (65, 6, 497), (511,), (2990, 6)])
+def test_resident_1d_split_over_ctas(built_lib, oracle_lib, sizes, bc):
+    """Sizes around the limits of the split of a block over the CTAs of a cluster (a warp of
+    interfaces each, at least six points, blocks of very different sizes together), perturbed
+    states: as the per-block path, halos included (1e-13: the same operations on the same values,
+    contracted differently at most), and FP32 against FP64 within 1e-5 after two steps."""
+    rng = np.random.default_rng(3)
+    blocks = []
+    for n in sizes:
+        spec, q = problems.sod(n, scheme=abi.SCHEME_TENO5, bc=BCS[bc])
+        blocks.append((spec, [a * (1.0 + 1e-2 * rng.standard_normal(a.shape)) for a in q]))
+    dt = 0.05 / max(sizes)
+    res, nl = _run(blocks, "ls3", dt, 2, None)
+    assert nl == 1
+    per, _ = _run(blocks, "ls3", dt, 2, abi.SCHED_PER_BLOCK)
+    from opensbli_gb300.solver import Solver
+    s = Solver(blocks, precision="fp32", rk="ls3")
+    s.apply_bc()
+    s.step(dt, 2)
+    f32 = [s.state(i) for i in range(len(blocks))]
+    s.close()
+    for i, (spec, _) in enumerate(blocks):
+        for v in range(spec.nvars):
+            assert harness.rel_err(res[i][v], per[i][v]) < 1e-13, (i, v)
+            assert harness.rel_err(f32[i][v], per[i][v]) < 1e-5, (i, v, "fp32")

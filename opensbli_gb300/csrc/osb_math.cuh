@@ -478,6 +478,36 @@ __device__ __forceinline__ void make_pt(Pt<double, ND>& s, double gm) {
   s.H = (s.q[ND + 1] + s.p) * ir;
 }
 
+// FP64 averaged state of an interface (averaging.py:31-124): velocity, sound speed and its
+// reciprocal, the average density squared, |u|^2.
+template <int ND, int AVG>
+__device__ __forceinline__ void face_average_f64(const Pt<double, ND>& L, const Pt<double, ND>& R, double g1,
+                                                 double (&u)[ND], double& a, double& ia, double& rho2, double& ke) {
+  ke = 0.0;
+  if (AVG == AVG_ROE) {
+    const double inv = rcp_newton(L.s + R.s), wl = L.s * inv, wr = R.s * inv;
+#pragma unroll
+    for (int i = 0; i < ND; ++i) {
+      u[i] = wl * L.u[i] + wr * R.u[i];
+      ke += u[i] * u[i];
+    }
+    const double a2 = g1 * (wl * L.H + wr * R.H - 0.5 * ke);
+    ia = rsqrt(a2);
+    a = a2 * ia;
+    rho2 = L.q[0] * R.q[0];
+  } else {
+#pragma unroll
+    for (int i = 0; i < ND; ++i) {
+      u[i] = 0.5 * (L.u[i] + R.u[i]);
+      ke += u[i] * u[i];
+    }
+    a = 0.5 * (L.a + R.a);
+    ia = rcp_newton(a);
+    const double rho = 0.5 * (L.q[0] + R.q[0]);
+    rho2 = rho * rho;
+  }
+}
+
 // FP64 characteristic LLF flux at the interface between w[2] and w[3] (the FP32 form and the
 // citations: char_flux), arranged for the fewest FP64 instructions.  With the averaged state u, a,
 // a point's projections are
@@ -502,30 +532,8 @@ __device__ __forceinline__ void char_flux_f64(const Pt<double, ND> (&w)[6], cons
   const double g1 = sp.g1;
   const Pt<double, ND>& L = w[2];
   const Pt<double, ND>& R = w[3];
-  double u[ND], a, ia, rho2;  // rho2: the average density squared
-  double ke = 0.0;
-  if (AVG == AVG_ROE) {
-    const double inv = rcp_newton(L.s + R.s), wl = L.s * inv, wr = R.s * inv;
-#pragma unroll
-    for (int i = 0; i < ND; ++i) {
-      u[i] = wl * L.u[i] + wr * R.u[i];
-      ke += u[i] * u[i];
-    }
-    const double a2 = g1 * (wl * L.H + wr * R.H - 0.5 * ke);
-    ia = rsqrt(a2);
-    a = a2 * ia;
-    rho2 = L.q[0] * R.q[0];
-  } else {
-#pragma unroll
-    for (int i = 0; i < ND; ++i) {
-      u[i] = 0.5 * (L.u[i] + R.u[i]);
-      ke += u[i] * u[i];
-    }
-    a = 0.5 * (L.a + R.a);
-    ia = rcp_newton(a);
-    const double rho = 0.5 * (L.q[0] + R.q[0]);
-    rho2 = rho * rho;
-  }
+  double u[ND], a, ia, rho2, ke;
+  face_average_f64<ND, AVG>(L, R, g1, u, a, ia, rho2, ke);
   const double hk = 0.5 * ke, gi = g1 * ia, g = gi * ia;
   const double lam_u = sp.sfc * fmax(fabs(L.u[0]), fabs(R.u[0]));
   const double lam_p = sp.sfc * fmax(fabs(L.u[0] + L.a), fabs(R.u[0] + R.a));

@@ -51,17 +51,19 @@ template <typename T>
 struct RLayout {
   double *q, *o;       // [3][most]: state and register
   double* halo;        // [2 parities][2 sides][RH points][3]: the neighbours' outer points
-  T *F;                // [3][most + 1]: flux at the left face of point i
+  T *F;                // [3][most + 1]: flux at the left face of point i (FP64: its three reconstructed waves)
+  T *V;                // FP64: [3][most + 1]: averaged u, a, 1 / a of the face
   T* P;                // [8][most + 2 RH]: rho, m, E, u, p, a (, sqrt(rho), H in FP64) from point -RH
   __device__ RLayout(unsigned char* sm, int most) {
     q = reinterpret_cast<double*>(sm);
     o = q + 3 * most;
     halo = o + 3 * most;
     F = reinterpret_cast<T*>(halo + 2 * 2 * RH * 3);
-    P = F + 3 * (most + 1);
+    V = F + 3 * (most + 1);
+    P = V + (sizeof(T) == 8 ? 3 * (most + 1) : 0);
   }
   static size_t bytes(int most) {
-    return sizeof(double) * (6 * (size_t)most + 2 * 2 * RH * 3) + sizeof(T) * (3 * (size_t)(most + 1) + 8 * (size_t)(most + 2 * RH));
+    return sizeof(double) * (6 * (size_t)most + 2 * 2 * RH * 3) + sizeof(T) * ((sizeof(T) == 8 ? 6 : 3) * (size_t)(most + 1) + 8 * (size_t)(most + 2 * RH));
   }
 };
 
@@ -90,24 +92,64 @@ __device__ __forceinline__ T to_t(double x) {
 }
 
 // Primitives of a point (make_pt) to and from its column of the staged arrays.
-template <typename T>
+template <typename T, int AVG>
 __device__ __forceinline__ void put_prims(T* P, int stride, const Pt<T, 1>& w) {
   P[3 * stride] = w.u[0];
   P[4 * stride] = w.p;
   P[5 * stride] = w.a;
-  if constexpr (sizeof(T) == 8) {
+  if constexpr (sizeof(T) == 8 && AVG == AVG_ROE) {
     P[6 * stride] = w.s;
     P[7 * stride] = w.H;
   }
 }
-template <typename T>
+template <typename T, int AVG>
 __device__ __forceinline__ void get_prims(const T* P, int stride, Pt<T, 1>& w) {
   w.u[0] = P[3 * stride];
   w.p = P[4 * stride];
   w.a = P[5 * stride];
-  if constexpr (sizeof(T) == 8) {
+  if constexpr (sizeof(T) == 8 && AVG == AVG_ROE) {
     w.s = P[6 * stride];
     w.H = P[7 * stride];
+  }
+}
+
+// FP64: the interfaces of a CTA are few (a warp of them), and an FP64 instruction's result takes
+// several times the 16 cycles of its issue, so one warp leaves the pipe mostly waiting.  Each
+// wave of an interface goes to its own warp (char_flux_f64's rows for one dimension): k = 0 entropy,
+// 1 u + a, 2 u - a.  The point's own thread turns the waves of its two faces into fluxes.
+template <int SCH>
+__device__ __forceinline__ double wave_1d(int k, const Pt<double, 1> (&w)[6], const SP<double>& sp, double u, double a,
+                                          double ia, double ke) {
+  const Pt<double, 1>& L = w[2];
+  const Pt<double, 1>& R = w[3];
+  const double hk = 0.5 * ke, gi = sp.g1 * ia, g = gi * ia;
+  const double sg = k == 0 ? 0.0 : (k == 1 ? 1.0 : -1.0);
+  const double lam = sp.sfc * fmax(fabs(__fma_rn(sg, L.a, L.u[0])), fabs(__fma_rn(sg, R.a, R.u[0])));
+  const double cp = k == 0 ? -g : gi;  // c = cp P + rho (entropy) or + sg D
+  double fp[6], fm[6];
+#pragma unroll
+  for (int m = 0; m < 6; ++m) {
+    const double P = __fma_rn(hk, w[m].q[0], __fma_rn(-u, w[m].q[1], w[m].q[2]));
+    const double D = k == 0 ? w[m].q[0] : sg * __fma_rn(-u, w[m].q[0], w[m].q[1]);
+    const double W = w[m].p * (w[m].u[0] - u);
+    const double c = __fma_rn(cp, P, D), t = __fma_rn(cp, W, sg * w[m].p);
+    fp[m] = __fma_rn(w[m].u[0] + lam, c, t);
+    fm[m] = __fma_rn(w[m].u[0] - lam, c, t);
+  }
+  const double s2 = k == 0 ? 4.0 : 16.0 * a * a;
+  if constexpr (SCH == SCH_TENO6) {
+    const double sc = k == 0 ? 2.0 : 4.0 * a, isc = k == 0 ? 0.5 : 0.25 * ia;
+#pragma unroll
+    for (int m = 0; m < 6; ++m) {
+      fp[m] *= isc;
+      fm[m] *= isc;
+    }
+    return sc * (recon6<double, 1>(fp[0], fp[1], fp[2], fp[3], fp[4], fp[5], sp) +
+                 recon6<double, -1>(fm[0], fm[1], fm[2], fm[3], fm[4], fm[5], sp));
+  } else {
+    const ReconEps e = recon_eps<SCH>(sp.teno_eps, s2);
+    return recon5_f64<SCH>(fp[0], fp[1], fp[2], fp[3], fp[4], e, sp.teno_ct, sp.teno_ct_f) +
+           recon5_f64<SCH>(fm[5], fm[4], fm[3], fm[2], fm[1], e, sp.teno_ct, sp.teno_ct_f);
   }
 }
 
@@ -188,17 +230,31 @@ __global__ void __launch_bounds__(RT) k_resident_1d(const Resident1D* __restrict
         T* P = L.P + i + RH;
 #pragma unroll
         for (int v = 0; v < 3; ++v) P[v * PS] = w.q[v];
-        put_prims(P, PS, w);
+        put_prims<T, AVG>(P, PS, w);
       }
       __syncthreads();
-      for (int i = threadIdx.x; i <= n; i += blockDim.x) {  // left face of point i
+      const int W = (n + 32) / 32 * 32;  // n + 1 faces, whole warps
+      for (int k = threadIdx.x; k < (F32 ? n + 1 : 3 * W); k += blockDim.x) {
+        const int wave = F32 ? 0 : k / W, i = k - wave * W;  // left face of point i
+        if (i > n) continue;
         Pt<T, 1> w[6];
 #pragma unroll
         for (int m = 0; m < 6; ++m) {
           const T* P = L.P + i + m;
 #pragma unroll
           for (int v = 0; v < 3; ++v) w[m].q[v] = P[v * PS];
-          get_prims(P, PS, w[m]);
+          get_prims<T, AVG>(P, PS, w[m]);
+        }
+        if constexpr (!F32) {
+          double u[1], a, ia, rho2, ke;
+          face_average_f64<1, AVG>(w[2], w[3], sp.g1, u, a, ia, rho2, ke);
+          L.F[wave * (most + 1) + i] = wave_1d<SCH>(wave, w, sp, u[0], a, ia, ke);
+          if (wave == 0) {
+            L.V[i] = u[0];
+            L.V[most + 1 + i] = a;
+            L.V[2 * (most + 1) + i] = ia;
+          }
+          continue;
         }
         T fh[3];
         char_flux<T, 1, SCH, AVG>(w, sp, fh);
@@ -209,9 +265,26 @@ __global__ void __launch_bounds__(RT) k_resident_1d(const Resident1D* __restrict
       const double A = rk.A[s], B = rk.B[s];
       const bool a_zero = rk.kind == 0 && A == 0.0;
       for (int i = threadIdx.x; i < n; i += blockDim.x) {
+        T face[2][3];
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const T* F = L.F + i + e;
+          if constexpr (F32) {
+#pragma unroll
+            for (int v = 0; v < 3; ++v) face[e][v] = F[v * (most + 1)];
+          } else {
+            const double* V = L.V + i + e;
+            const double u = V[0], a = V[most + 1], ia = V[2 * (most + 1)];
+            const double r0 = 0.5 * F[0], rp = F[most + 1], rm = F[2 * (most + 1)];
+            const double S = 0.25 * (rp + rm), Bm = 0.25 * (rp - rm), F0 = __fma_rn(ia, S, r0);
+            face[e][0] = F0;
+            face[e][1] = __fma_rn(u, F0, Bm);
+            face[e][2] = __fma_rn(0.5 * (u * u), F0, __fma_rn(a * sp.ig1, S, u * Bm));
+          }
+        }
 #pragma unroll
         for (int v = 0; v < 3; ++v) {
-          const T fl = L.F[v * (most + 1) + i], fr = L.F[v * (most + 1) + i + 1];
+          const T fl = face[0][v], fr = face[1][v];
           double ov = L.o[v * most + i], qv = L.q[v * most + i];
           if constexpr (F32) {
             float p, pe;
@@ -308,7 +381,8 @@ int launch_resident(osb_ctx* c, const Resident1D* dev, int nblocks, int maxN, do
     at.val.clusterDim.x = (unsigned)C;
     at.val.clusterDim.y = at.val.clusterDim.z = 1;
     cfg.gridDim = dim3((unsigned)(nblocks * C));
-    cfg.blockDim = dim3((unsigned)std::min(RT, (most + 2 * RH + 31) / 32 * 32));
+    const int W = (most + 32) / 32 * 32;
+    cfg.blockDim = dim3((unsigned)std::min(RT, sizeof(T) == 8 ? 3 * W : (most + 2 * RH + 31) / 32 * 32));
     cfg.dynamicSmemBytes = smem;
     if (C <= 8) break;  // a portable cluster size
     int granted = 0;

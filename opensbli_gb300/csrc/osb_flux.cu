@@ -25,14 +25,16 @@ namespace {
 template <typename T, int ND, int D, int SCH, int AVG, bool CURV, bool FUSE, int FLX>
 int launch_sweep_k(osb_ctx* c, const BlockK& k, const SchemeParams& sp, int N, int other, const RkFuse& rf) {
   auto kern = k_flux_sweep<T, ND, D, SCH, AVG, CURV, FUSE, FLX>;
-  const long slots = (long)resident_ctas(kern, SWEEP_THREADS, 0) * c->sm_count;
+  constexpr size_t smem = sweep_smem<T, ND, CURV, FUSE>();
+  OSB_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const long slots = (long)resident_ctas(kern, SWEEP_THREADS, smem) * c->sm_count;
   const long gx = ((long)k.n[0] * other + SWEEP_THREADS - 1) / SWEEP_THREADS;
   int nseg = wave_chunks(N, gx, slots, 1.5, 8);
   const int seg = (N + nseg - 1) / nseg;
   nseg = (N + seg - 1) / seg;
   if (other > 65535 || nseg > 65535) return fail(OSB_ENOTSUP, "block too large for the sweep grid");
   dim3 grid((unsigned)gx, (unsigned)nseg);
-  kern<<<grid, SWEEP_THREADS, 0, c->stream>>>(k, sp, seg, nseg, 0, rf);
+  kern<<<grid, SWEEP_THREADS, smem, c->stream>>>(k, sp, seg, nseg, 0, rf);
   return OSB_OK;
 }
 

@@ -754,7 +754,7 @@ int timing_collect(osb_ctx* c) {
 
 // Residual kernels of one block.  With rf (FP32 path) the last of them applies the RK update
 // itself (*fused = true): the central kernel when there is one, else the last sweep of a 2D/3D
-// block.
+// block with the LLF flux.
 template <typename T>
 int residual_t(osb_ctx* c, Block& bl, const RkFuse* rf, bool* fused) {
   SchemeParams sp = scheme_params(bl.d.gama, bl.d.eps, bl.d.teno_ct, bl.d.shock_filter_control, 1e-12);
@@ -767,11 +767,11 @@ int residual_t(osb_ctx* c, Block& bl, const RkFuse* rf, bool* fused) {
   } else {
     const int nd = bl.d.ndim;
     const bool visc = bl.d.viscous != OSB_VISC_NONE;
-    // the last sweep of a 3D Cartesian block carries the update (z sweep + update 4.34 against
-    // 4.53 ms per step of the 256^3 Euler TGV with the separate k_rk32); the curvilinear sweeps
-    // (168 registers) do not: there the extra FP64 state and register loads are not hidden
-    // (5.60 against 5.01 ms per step of the 4-block case), nor in 2D, which is unmeasured
-    const RkFuse* rs = (sizeof(T) == 4 && !visc && nd == 3 && !bl.k.m[9]) ? rf : nullptr;
+    // The last sweep of a 2D / 3D Euler block carries the update: with the state and register in the
+    // sweep's cp.async ring, z sweep and update of the 4-block curvilinear case take 3.72 ms a step
+    // against 2.68 + 1.67 with k_rk32.  A viscous block leaves it to the central kernel: there the
+    // update costs 0.32 ms of the 256^3 block's stage, in the z sweep 0.38.
+    const RkFuse* rs = (sizeof(T) == 4 && !visc && nd >= 2 && bl.d.flux_type == OSB_FLUX_LLF) ? rf : nullptr;
     if (bl.k.m[9]) {
       if (sizeof(T) == 4) rc = nd == 2 ? flux_curv_f32_2d(c, bl, sp, rs) : flux_curv_f32_3d(c, bl, sp, rs);
       else rc = nd == 2 ? flux_curv_f64_2d(c, bl, sp, nullptr) : flux_curv_f64_3d(c, bl, sp, nullptr);

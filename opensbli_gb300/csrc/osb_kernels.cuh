@@ -362,6 +362,14 @@ __device__ __forceinline__ int gvar(int lv) {
 // with 20 (spilling); 0.79 before the packed flux.  The curvilinear z sweep of the 4-block case
 // takes 0.22 ms instead of 0.29.
 constexpr int SWEEP_THREADS = 128, SWEEP_RING = 3;
+// FUSE: the ring also carries the point's FP64 state and RK register, so the update's 80 bytes per
+// point arrive under the arithmetic.
+template <typename T, int ND, bool CURV, bool FUSE>
+constexpr size_t sweep_smem() {
+  return (size_t)SWEEP_RING * SWEEP_THREADS *
+         (sizeof(T) * (SweepFields<ND, CURV>::N + (sizeof(T) == 4 ? 2 : 1) * (ND + 2)) +
+          (FUSE ? sizeof(double) * 2 * (ND + 2) : 0));
+}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_prev() { asm volatile("cp.async.wait_group 1;\n" ::: "memory"); }
 
@@ -373,7 +381,10 @@ __global__ void __launch_bounds__(SWEEP_THREADS, sizeof(T) == 4 ? 3 : 1)
   constexpr int NR = sizeof(T) == 4 ? 2 * NV : NV;  // residual words of a point: float-float pairs or doubles
   constexpr int NS = NF + NR;
   using P = typename SweepPt<T, ND, CURV>::type;
-  __shared__ T ring[SWEEP_RING][NS][SWEEP_THREADS];
+  extern __shared__ __align__(16) unsigned char osb_smem[];
+  double (*upd)[2 * NV][SWEEP_THREADS] = reinterpret_cast<double (*)[2 * NV][SWEEP_THREADS]>(osb_smem);  // FUSE only
+  T (*ring)[NS][SWEEP_THREADS] =
+      reinterpret_cast<T (*)[NS][SWEEP_THREADS]>(osb_smem + (FUSE ? sizeof(double) * SWEEP_RING * 2 * NV * SWEEP_THREADS : 0));
   const SP<T> sp(spd);
   const int tid = threadIdx.x;
   // the block's lines (x, transverse) are one index space, so rows of any length fill the warps:
@@ -408,6 +419,10 @@ __global__ void __launch_bounds__(SWEEP_THREADS, sizeof(T) == 4 ? 3 : 1)
           cp_async_el(&ring[slot][NF + 2 * lv + 1][tid], b.Rl[v] + idr);
         } else {
           cp_async_el(&ring[slot][NF + lv][tid], b.R[v] + idr);
+        }
+        if constexpr (FUSE) {
+          cp_async_el(&upd[slot][lv][tid], b.q[v] + idr);
+          if (!rf.a_zero) cp_async_el(&upd[slot][NV + lv][tid], b.rk[v] + idr);
         }
       }
     }
@@ -468,7 +483,8 @@ __global__ void __launch_bounds__(SWEEP_THREADS, sizeof(T) == 4 ? 3 : 1)
 #pragma unroll
         for (int lv = 0; lv < NV; ++lv) {
           r_final(fh[lv], fprev[lv], sc, oh[lv], ol[lv]);
-          nbad += rk_point(b, rf, gvar<ND, D, CURV>(lv), id, oh[lv], ol[lv]);
+          nbad += rk_point_ff(b, rf, gvar<ND, D, CURV>(lv), id, oh[lv], ol[lv], upd[cur][lv][tid],
+                              rf.a_zero ? 0.0 : upd[cur][NV + lv][tid]);
         }
       } else if (first) {
 #pragma unroll

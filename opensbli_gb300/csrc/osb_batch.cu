@@ -168,7 +168,7 @@ __global__ void __launch_bounds__(BTHREADS, 2) k_batch2d(const BatchBlock* __res
         float h = __fadd_rn(p1, e1);
         float l = __fsub_rn(e1, __fsub_rn(h, p1));
         ff_add(h, l, p2, e2);
-        const double x = dt_residual(h, l, dt_h, dt_l);  // as rk_point_ff
+        const double x = dt_residual(h, l, dt_h, dt_l);  // as rk_point
         double q = bk.q[v][id];
         double o;
         if (kind == 0) {

@@ -2,7 +2,7 @@
 // once per precision (OSB_CENTRAL_T).
 #include "osb_closures.h"
 #include "osb_internal.h"
-#include "osb_central64.cuh"
+#include "osb_central_tile.cuh"
 
 #include <algorithm>
 #include <cmath>
@@ -59,61 +59,42 @@ CentralParams central_params(const Block& bl) {
   return cp;
 }
 
-template <typename T, int CONV, int VISC, bool FUSE, int CY, bool BULK, bool WALL = false>
-int launch_central_k(osb_ctx* c, Block& bl, int first, const RkFuse& rf) {
-  using Fd = CentralFields<T, CONV, VISC>;
-  size_t smem = (size_t)Fd::N * CRING * CTile<CY, WALL ? 4 : CH>::CPL * sizeof(T);
-  if (BULK) smem += CTile<CY>::RAW * sizeof(float) + 2 * sizeof(unsigned long long);
-  auto kern = k_central3d<T, CONV, VISC, FUSE, CY, BULK, WALL>;
-  OSB_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  const CentralParams cp = central_params<WALL>(bl);
-  const BlockK& k = bl.k;
-  // z chunks per column: whole waves of resident CTAs; a chunk starts by staging four planes
-  // (two of halo) at about a third of the cost of a computed plane each
-  const long cols = (long)((k.n[0] + CX - 1) / CX) * ((k.n[1] + CY - 1) / CY);
-  const long slots = (long)resident_ctas(kern, CX * CY, smem) * c->sm_count;
-  const int nz = wave_chunks(k.n[2], cols, slots, 1.4, 4);
+// Launch shape of a kernel on 32 x rows columns: z chunks per column so the CTAs fill whole waves (a
+// chunk starts by staging four planes, `start` computed planes' worth).
+struct ColumnGrid {
+  dim3 grid;
+  int czc;
+};
+template <typename K>
+ColumnGrid column_grid(osb_ctx* c, const BlockK& k, K kern, int rows, size_t smem, double start) {
+  const unsigned nx = (k.n[0] + CX - 1) / CX, ny = (k.n[1] + rows - 1) / rows;
+  const long slots = (long)resident_ctas(kern, CX * rows, smem) * c->sm_count;
+  const int nz = wave_chunks(k.n[2], (long)nx * ny, slots, start, 4);
   const int czc = (k.n[2] + nz - 1) / nz;
-  dim3 grid((k.n[0] + CX - 1) / CX, (k.n[1] + CY - 1) / CY, (k.n[2] + czc - 1) / czc);
+  return {dim3(nx, ny, (k.n[2] + czc - 1) / czc), czc};
+}
+
+template <typename T, int VISC, bool FUSE>
+int launch_wall(osb_ctx* c, Block& bl, int first, const RkFuse& rf) {
+  auto kern = k_central_wall<T, VISC, FUSE>;
+  constexpr size_t smem = (size_t)WallFields::N * CRING * CPL * sizeof(T);
+  OSB_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const ColumnGrid g = column_grid(c, bl.k, kern, CWY, smem, 1.4);
   timing_begin(c, FAM_CENTRAL);
-  kern<<<grid, CX * CY, smem, c->stream>>>(k, cp, first, czc, rf);
+  kern<<<g.grid, CX * CWY, smem, c->stream>>>(bl.k, central_params<true>(bl), first, g.czc, rf);
   timing_end(c);
   c->launches++;
   return OSB_OK;
 }
 
-// Tile height of the FP32 kernels: 8 rows unless the ring holds the KGP form's eleven fields of a
-// block whose cross-section already gives every SM several columns (measured: 8 rows are 37 %
-// faster on the 64^3 central TGV and equal on the 256^3 TENO5 one; 4 rows are 1.4 % faster for
-// the 256^3 KGP form).  FP64 (the KGP form alone, FP64-pipe bound, a ring twice as large): 4 rows.
 template <typename T, int CONV, int VISC, bool FUSE, bool BULK>
-int launch_central_h(osb_ctx* c, Block& bl, int first, const RkFuse& rf) {
-  if constexpr (CONV == 0 && !BULK) {
-    if (is_wall(bl.d.bc[1][0]) || is_wall(bl.d.bc[1][1]))
-      return launch_central_k<T, CONV, VISC, FUSE, 4, false, true>(c, bl, first, rf);
-  }
-  const long cols4 = (long)((bl.k.n[0] + CX - 1) / CX) * ((bl.k.n[1] + 3) / 4);
-  if (sizeof(T) == 8 || (CONV == 2 && cols4 >= 2L * c->sm_count))
-    return launch_central_k<T, CONV, VISC, FUSE, 4, BULK>(c, bl, first, rf);
-  if constexpr (sizeof(T) == 4) return launch_central_k<T, CONV, VISC, FUSE, 8, BULK>(c, bl, first, rf);
-  return OSB_OK;
-}
-
-// FP64 blocks without wall faces: Feiereisen and viscous terms (k_central_f64).
-template <int CONV, int VISC>
-int launch_central_f64(osb_ctx* c, Block& bl, int first) {
-  auto kern = k_central_f64<CONV, VISC>;
-  constexpr size_t smem = c64_smem<CONV, VISC>();
+int launch_tile(osb_ctx* c, Block& bl, int first, const RkFuse& rf) {
+  auto kern = k_central<T, CONV, VISC, FUSE, BULK>;
+  constexpr size_t smem = ct_smem<T, CONV, VISC, FUSE, BULK>();
   OSB_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  const BlockK& k = bl.k;
-  const long cols = (long)((k.n[0] + CX - 1) / CX) * ((k.n[1] + C64Y - 1) / C64Y);
-  const long slots = (long)resident_ctas(kern, C64T, smem) * c->sm_count;
-  // a chunk's four planes of start-up cost their staging, about a fifth of a computed plane each
-  const int nz = wave_chunks(k.n[2], cols, slots, 0.9, 4);
-  const int czc = (k.n[2] + nz - 1) / nz;
-  dim3 grid((k.n[0] + CX - 1) / CX, (k.n[1] + C64Y - 1) / C64Y, (k.n[2] + czc - 1) / czc);
+  const ColumnGrid g = column_grid(c, bl.k, kern, CTY, smem, sizeof(T) == 8 ? 0.9 : 1.4);
   timing_begin(c, FAM_CENTRAL);
-  kern<<<grid, C64T, smem, c->stream>>>(k, central_params<false>(bl), first, czc);
+  kern<<<g.grid, CTT, smem, c->stream>>>(bl.k, central_params<false>(bl), first, g.czc, rf);
   timing_end(c);
   c->launches++;
   return OSB_OK;
@@ -123,18 +104,19 @@ int launch_central_f64(osb_ctx* c, Block& bl, int first) {
 // planes come in by register loads or, after osb_set_central_staging(1), by bulk copies.
 template <typename T, int CONV, int VISC>
 int launch_central_t(osb_ctx* c, Block& bl, int first, const RkFuse* rf) {
-  const bool wall = is_wall(bl.d.bc[1][0]) || is_wall(bl.d.bc[1][1]);
-  if constexpr (sizeof(T) == 8 && CONV != 2) {
-    if (!wall) return launch_central_f64<CONV, VISC>(c, bl, first);
-    if constexpr (CONV == 0) return launch_central_k<T, 0, VISC, false, 4, false, true>(c, bl, first, RkFuse{});
-    return fail(OSB_ENOTSUP, "walls are implemented for shock-capturing schemes");
-  } else {
-    if constexpr (sizeof(T) == 4) {
-      if (rf && c->central_bulk && !wall) return launch_central_h<T, CONV, VISC, true, true>(c, bl, first, *rf);
-      if (rf) return launch_central_h<T, CONV, VISC, true, false>(c, bl, first, *rf);
+  if (is_wall(bl.d.bc[1][0]) || is_wall(bl.d.bc[1][1])) {
+    if constexpr (CONV == 0 && VISC != 0) {
+      if constexpr (sizeof(T) == 4)
+        if (rf) return launch_wall<T, VISC, true>(c, bl, first, *rf);
+      return launch_wall<T, VISC, false>(c, bl, first, RkFuse{});
     }
-    return launch_central_h<T, CONV, VISC, false, false>(c, bl, first, RkFuse{});
+    return fail(OSB_ENOTSUP, "walls are implemented for shock-capturing schemes");
   }
+  if constexpr (sizeof(T) == 4) {
+    if (rf && c->central_bulk) return launch_tile<T, CONV, VISC, true, true>(c, bl, first, *rf);
+    if (rf) return launch_tile<T, CONV, VISC, true, false>(c, bl, first, *rf);
+  }
+  return launch_tile<T, CONV, VISC, false, false>(c, bl, first, RkFuse{});
 }
 
 template <typename T>

@@ -84,7 +84,11 @@ __global__ void k_rk32(BlockK b, int nv, RkFuse rf) {
     int j = r % b.n[1];
     int k = r / b.n[1];
     int id = lin(b, i, j, k);
-    for (int v = 0; v < nv; ++v) nb += rk_point(b, rf, v, id, b.Rh[v][id], b.Rl[v][id]);
+    rk_modes(rf, [&](auto mode) {
+      constexpr int MODE = decltype(mode)::value;
+      for (int v = 0; v < nv; ++v)
+        nb += rk_point<MODE>(b, rf, v, id, b.Rh[v][id], b.Rl[v][id], b.q[v][id], MODE == 0 ? 0.0 : b.rk[v][id]);
+    });
   }
   if (nb) atomicAdd(rf.bad, (unsigned long long)nb);
 }

@@ -285,35 +285,36 @@ __device__ __forceinline__ double dt_residual(float h, float l, float dt_h, floa
 }
 
 // RK update of one variable from the float-float residual (h, l) with x = dt_residual: two
-// FP64 FMAs, the register and the state (rk_LS.py:204-215; rk_sbli.py:138-145).
-__device__ __forceinline__ unsigned rk_point_ff(const BlockK& b, const RkFuse& rf, int v, int id, float h, float l,
-                                                double q, double o) {
+// FP64 FMAs, the register and the state (rk_LS.py:204-215; rk_sbli.py:138-145).  MODE: 0 the first
+// low-storage stage (A = 0: the register becomes x, one FMA), 1 low-storage, 2 SBLI.
+template <int MODE>
+struct RkMode {
+  static constexpr int value = MODE;
+};
+template <int MODE>
+__device__ __forceinline__ unsigned rk_point(const BlockK& b, const RkFuse& rf, int v, int id, float h, float l,
+                                             double q, double o) {
   const double x = dt_residual(h, l, rf.dt_h, rf.dt_l);
-  if (rf.kind == 0) {
-    o = rf.a_zero ? x : __fma_rn(rf.A, o, x);
-    q = __fma_rn(rf.B, o, q);
-  } else {
+  if (MODE == 2) {
     q = __fma_rn(rf.A, x, o);
     o = __fma_rn(rf.B, x, o);
+  } else {
+    o = MODE == 0 ? x : __fma_rn(rf.A, o, x);
+    q = __fma_rn(rf.B, o, q);
   }
   b.rk[v][id] = o;
   b.q[v][id] = q;
   rf.qout[v][id] = d2f_rn(q);
   return ((((unsigned)__double2hiint(q) >> 20) & 0x7ffu) == 0x7ffu) ? 1u : 0u;
 }
-// The first low-storage stage (A = 0): the register becomes x, one FP64 FMA.  Callers take
-// this path under a uniform branch; the select in rk_point_ff gives the same values.
-__device__ __forceinline__ unsigned rk_point_a0(const BlockK& b, const RkFuse& rf, int v, int id, float h, float l,
-                                                double q) {
-  const double x = dt_residual(h, l, rf.dt_h, rf.dt_l);
-  q = __fma_rn(rf.B, x, q);
-  b.rk[v][id] = x;
-  b.q[v][id] = q;
-  rf.qout[v][id] = d2f_rn(q);
-  return ((((unsigned)__double2hiint(q) >> 20) & 0x7ffu) == 0x7ffu) ? 1u : 0u;
-}
-__device__ __forceinline__ unsigned rk_point(const BlockK& b, const RkFuse& rf, int v, int id, float h, float l) {
-  return rk_point_ff(b, rf, v, id, h, l, b.q[v][id], rf.a_zero ? 0.0 : b.rk[v][id]);
+// Runs f with the launch's mode: a branch around all of a point's variables.  Selecting between the
+// modes per variable instead evaluates both and takes twice the FP64 FMAs (the pipe was 50 % busy in
+// the fused central kernel, for 10 FMAs per point).
+template <typename Fn>
+__device__ __forceinline__ void rk_modes(const RkFuse& rf, Fn f) {
+  if (rf.kind != 0) f(RkMode<2>{});
+  else if (rf.a_zero) f(RkMode<0>{});
+  else f(RkMode<1>{});
 }
 
 // Final residual of a point (float-float) from its prefetched partial value plus the last
@@ -480,12 +481,15 @@ __global__ void __launch_bounds__(SWEEP_THREADS, sizeof(T) == 4 ? 3 : 1)
       if constexpr (D == 1 && !CURV)
         if (b.ys[0]) sc = invd * ystr<T>(b, 0, j);
       if constexpr (FUSE) {
+        rk_modes(rf, [&](auto mode) {
+          constexpr int MODE = decltype(mode)::value;
 #pragma unroll
-        for (int lv = 0; lv < NV; ++lv) {
-          r_final(fh[lv], fprev[lv], sc, oh[lv], ol[lv]);
-          nbad += rk_point_ff(b, rf, gvar<ND, D, CURV>(lv), id, oh[lv], ol[lv], upd[cur][lv][tid],
-                              rf.a_zero ? 0.0 : upd[cur][NV + lv][tid]);
-        }
+          for (int lv = 0; lv < NV; ++lv) {
+            r_final(fh[lv], fprev[lv], sc, oh[lv], ol[lv]);
+            nbad += rk_point<MODE>(b, rf, gvar<ND, D, CURV>(lv), id, oh[lv], ol[lv], upd[cur][lv][tid],
+                                   MODE == 0 ? 0.0 : upd[cur][NV + lv][tid]);
+          }
+        });
       } else if (first) {
 #pragma unroll
         for (int lv = 0; lv < NV; ++lv) acc_flux(b, gvar<ND, D, CURV>(lv), id, fh[lv], fprev[lv], sc, 1);
@@ -651,13 +655,6 @@ __global__ void __launch_bounds__(32 * XWARPS, sizeof(T) == 4 ? 6 : 1) k_flux_x(
 }
 
 // ---------------------------------------------------------------------------------------
-// Central 4th-order terms on a 3D tile (CX x CY x CZ points, halo 2 with edges).
-//   CONV: central convective terms, 1 = skew-symmetric (Feiereisen) form, split_forms.py:111-145
-//         as generated for the low-Mach TGV ("Convective terms" kernel); 2 = Kennedy-Gruber-
-//         Pirozzoli form, split_forms.py:178-236 as generated for the Central4-WENO5 benchmark
-//         (its ring holds H = (rhoE + p) / rho where form 1 holds rhoE).
-//   VISC: viscous stress and heat flux (StoreSome "Viscous terms" kernel), mu from the
-//         modified Sutherland law (VISC == 1) or constant (VISC == 2).
 // Constants of the central kernel, derived once on the host in FP64 and handed over in both
 // precisions (a conversion or division in FP64 inside an FP32 kernel runs on the FP64 pipe).
 struct CentralParams {
@@ -684,31 +681,9 @@ __device__ __forceinline__ double cpar<double>(double d, float) { return d; }
 template <>
 __device__ __forceinline__ float cpar<float>(double, float f) { return f; }
 
-// A CTA owns a 32 x CY column of points and streams it through czc planes of z (a launch
-// argument, chosen on the host so the CTAs fill whole waves): the planes
-// z-2 .. z+2 around the current one sit in a 5-plane ring in shared memory (halo 2 in x and y,
-// edges included), the raw state of plane z+3 is loaded into registers while plane z is
-// computed, then converted to primitives into the slot plane z-2 vacates.
-// The tile height CY is a template argument: 8 rows stage fewer halo points per computed point
-// (36 x 12 / 256 against 36 x 8 / 128) and give small blocks more threads per column, 4 rows keep
-// the shared-memory ring small when it holds many fields (the KGP form with viscous terms).
-// BULK (FP32 state only): the raw planes come in through the bulk-copy (TMA) engine instead --
-// one cp.async.bulk per staged row and variable into a two-slot raw buffer in shared memory,
-// completion counted on an mbarrier per slot, two planes ahead of the computed one.  The OPS
-// row pitch (n + 10 elements) is not a multiple of 16 bytes, which a tiled tensor map needs,
-// so each row copy starts at the 16-byte boundary at or below the row's first staged element
-// and moves CRW elements; the lead (0..3 elements) is recomputed by the reading thread.
 constexpr int CX = 32, CH = 2, CRING = 5;
 constexpr int CSX = CX + 2 * CH;
 constexpr int CRW = 40;  // elements per bulk row copy: CSX plus a lead of up to 3, in 16-byte units
-template <int CY, int HY = CH>
-struct CTile {
-  static constexpr int CSY = CY + 2 * HY;  // HY: staged rows above and below the tile
-  static constexpr int CPL = CSX * CSY;                        // points of one staged plane
-  static constexpr int CPP = (CPL + CX * CY - 1) / (CX * CY);  // staged points per thread and plane
-  static constexpr int RAW = 2 * 5 * CSY * CRW;                // floats of the two raw plane slots
-};
-
 // ---- bulk-copy (TMA) staging: mbarrier and cp.async.bulk wrappers ----
 __device__ __forceinline__ unsigned smem_addr(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void mbar_init(unsigned long long* bar, unsigned count) {
@@ -754,40 +729,25 @@ __device__ __forceinline__ void bulk_copy_g2s(void* dst, const void* src, unsign
                : "memory");
 }
 
-template <typename T, int CONV, int VISC>
-struct CentralFields {
-  // indices into the shared-memory field array
-  static constexpr int U0 = 0, U1 = 1, U2 = 2, P = 3;
-  static constexpr int TT = 4, MU = 5;
-  static constexpr int RHO = VISC ? 6 : 4, M0 = RHO + 1, M1 = RHO + 2, M2 = RHO + 3, E = RHO + 4;
-  static constexpr int N = CONV ? (VISC ? 11 : 9) : 6;
+// Viscous terms of a shock-capturing block with isothermal or adiabatic wall y faces (cp.wall_lo /
+// cp.wall_hi), optionally on a stretched y grid (the other blocks: k_central).  A CTA owns a 32 x 4
+// column of points, streamed through z with a 5-plane ring like k_central's; it stages 4 rows above and
+// below instead of 2, and the y derivatives of the points next to a wall take the one-sided closures.
+constexpr int CWY = 4, CHY = 4;                          // tile height, staged rows above and below
+constexpr int CSY = CWY + 2 * CHY, CPL = CSX * CSY;      // staged rows, points of one staged plane
+constexpr int CPP = (CPL + CX * CWY - 1) / (CX * CWY);   // staged points per thread and plane
+struct WallFields {
+  static constexpr int U0 = 0, U1 = 1, U2 = 2, P = 3, TT = 4, MU = 5, N = 6;
 };
 
-// BULK: at least as many CTAs per SM as its shared memory (ring, raw slots, mbarriers; 228 KB per
-// SM, 1 KB reserved per CTA) admits, so the register allocation does not lower the occupancy.
-// Without BULK the minimum is 0 (none declared): an explicit 1 lets the compiler spend twice the
-// registers at half the occupancy.
-template <int NF, int CY, bool BULK>
-constexpr int bulk_ctas() {
-  return BULK ? (228 * 1024) / (NF * CRING * CTile<CY>::CPL * 4 + CTile<CY>::RAW * 4 + 16 + 1024) : 0;
-}
-// WALL: isothermal-wall y faces (cp.wall_lo / cp.wall_hi) -- the tile stages 4 rows above and
-// below instead of 2, and the y derivatives of the points next to a wall take the one-sided
-// closures (viscous terms of a shock-capturing block; CONV == 0).
-template <typename T, int CONV, int VISC, bool FUSE, int CY, bool BULK = false, bool WALL = false>
-__global__ void __launch_bounds__(CX * CY, bulk_ctas<CentralFields<T, CONV, VISC>::N, CY, BULK>()) k_central3d(BlockK b, CentralParams cp, int first, int czc, RkFuse rf) {
-  static_assert(!BULK || (sizeof(T) == 4 && FUSE), "bulk staging: FP32 state, fused update (error counter)");
-  static_assert(!WALL || (CONV == 0 && !BULK), "wall closures: viscous terms of shock-capturing blocks");
-  constexpr int CHY = WALL ? 4 : CH;  // staged rows above and below the tile
-  constexpr int CPL = CTile<CY, CHY>::CPL, CPP = CTile<CY, CHY>::CPP, CSY = CTile<CY, CHY>::CSY;
-  using Fd = CentralFields<T, CONV, VISC>;
+template <typename T, int VISC, bool FUSE>
+__global__ void __launch_bounds__(CX * CWY) k_central_wall(BlockK b, CentralParams cp, int first, int czc, RkFuse rf) {
+  constexpr int CY = CWY;
+  constexpr bool WALL = true;
+  using Fd = WallFields;
   constexpr int FS = CRING * CPL;  // field stride in shared memory
   extern __shared__ __align__(16) unsigned char osb_smem[];
   T* sm = reinterpret_cast<T*>(osb_smem);
-  // BULK: raw plane slots after the ring (16-byte aligned: FS * 4 bytes is a multiple of 16),
-  // then one mbarrier per slot
-  float* raw = reinterpret_cast<float*>(sm + Fd::N * FS);
-  unsigned long long* bar = reinterpret_cast<unsigned long long*>(raw + CTile<CY>::RAW);
   const int tx = threadIdx.x % CX, ty = threadIdx.x / CX;
   const int x0 = blockIdx.x * CX, y0 = blockIdx.y * CY;
   const int zb = blockIdx.z * czc, ze = min(b.n[2], zb + czc);
@@ -834,109 +794,15 @@ __global__ void __launch_bounds__(CX * CY, bulk_ctas<CentralFields<T, CONV, VISC
                                                               : L_(1.4042) * Tt * sqrt(Tt) / (L_(0.40417) + Tt))
                                            : mu_c;
       }
-      if (CONV) {
-        sm[Fd::RHO * FS + at] = rho;
-        sm[Fd::M0 * FS + at] = m0;
-        sm[Fd::M1 * FS + at] = m1;
-        sm[Fd::M2 * FS + at] = m2;
-        sm[Fd::E * FS + at] = CONV == 2 ? (E + p) / rho : E;
-      }
     }
   };
   auto slot_of = [](int gz) { return (gz + 2 * CRING) % CRING; };
-  // BULK: plane gz goes to raw slot (gz - zb + CH) & 1 and completes that slot's phase of
-  // parity ((gz - zb + CH) >> 1) & 1; rows past y = n1 + CH are not copied.  A wait that runs
-  // out marks the CTA broken (uniformly, through the next barrier): it issues no further copies,
-  // counts the event in *rf.stall, and before returning waits (bounded) for the copies it issued.
-  const int nrow = min(CSY, b.n[1] + 2 * CH + 1 - y0);
-  bool broken = false;
-  unsigned pend = 0, ppar = 0;  // raw slots with a copy in flight no wait has seen complete, its parity
-  auto rslot = [&](int gz) { return (gz - zb + CH) & 1; };
-  auto rpar = [&](int gz) { return (unsigned)((gz - zb + CH) >> 1) & 1u; };
-  // The copies of a plane are spread over lanes 0..7 of every warp (one warp issuing all of them
-  // measured 10 % slower); thread 0 arms the slot's next phase (arrive + expected bytes) as soon
-  // as its wait saw the previous one complete, so the copies need no extra barrier.
-  const unsigned plane_bytes = (unsigned)(nrow * 5 * CRW * 4);
-  auto issue = [&](int gz) {  // the bookkeeping is uniform
-    if (!BULK || broken || gz > ze + CH - 1) return;
-    const int s = rslot(gz);
-    pend |= 1u << s;
-    ppar = (ppar & ~(1u << s)) | (rpar(gz) << s);
-    const int lane = threadIdx.x & 31;
-    if (lane >= 8) return;
-    fence_async_smem();
-    for (int c = (threadIdx.x >> 5) * 8 + lane; c < 5 * nrow; c += CY * 8) {
-      const int v = c / nrow, r = c - v * nrow;
-      const float* src = b.qf[v] + lin(b, x0 - CH, y0 - CH + r, gz);
-      const float* al = reinterpret_cast<const float*>(reinterpret_cast<size_t>(src) & ~(size_t)15);
-      bulk_copy_g2s(raw + ((s * 5 + v) * CSY + r) * CRW, al, CRW * 4, &bar[s]);
-    }
-  };
-  // the 16-byte phase (0..3 elements) of each variable's array, two bits per variable: a row
-  // copy's lead is that phase plus the row's linear index, mod 4
-  unsigned phase = 0;
-  if constexpr (BULK) {
-#pragma unroll
-    for (int v = 0; v < 5; ++v) phase |= (unsigned)((reinterpret_cast<size_t>(b.qf[v]) >> 2) & 3) << (2 * v);
+  // prologue: planes zb-2 .. zb+1 into the ring, plane zb+2 into registers
+  for (int gz = zb - CH; gz < zb + CH; ++gz) {
+    load_plane(gz);
+    store_plane(slot_of(gz));
   }
-  // raw plane gz from its slot into the registers of the staged points (waits for the copy)
-  auto fetch_plane = [&](int gz) -> int {
-    const int s = rslot(gz);
-    int late = 0;
-    if (!broken) {
-      late = mbar_wait_bounded(&bar[s], rpar(gz)) ? 0 : 1;
-      if (!late) pend &= ~(1u << s);
-      if (!late && threadIdx.x == 0 && gz + 2 <= ze + CH - 1) mbar_arrive_expect(&bar[s], plane_bytes);
-    }
-#pragma unroll
-    for (int u = 0; u < CPP; ++u) {
-      const int idx = threadIdx.x + u * CX * CY;
-      const int ry = idx / CSX, cx = idx % CSX;
-      if (idx < CPL && x0 - CH + cx <= b.n[0] + CH && y0 - CH + ry <= b.n[1] + CH) {
-        const unsigned rl = (unsigned)lin(b, x0 - CH, y0 - CH + ry, gz);
-        const float* rrow = raw + (s * 5 * CSY + ry) * CRW + cx;
-#pragma unroll
-        for (int v = 0; v < 5; ++v) qv[u][v] = rrow[v * CSY * CRW + (int)(((phase >> (2 * v)) + rl) & 3u)];
-      }
-    }
-    return late;
-  };
-  // the barrier after a staged plane; BULK: also makes `broken` uniform
-  auto plane_barrier = [&](int late) {
-    if constexpr (BULK) {
-      const bool was = broken;
-      broken = __syncthreads_or(late) != 0 || was;
-      if (broken && !was && threadIdx.x == 0) atomicAdd(rf.stall, 1ull);
-    } else {
-      __syncthreads();
-    }
-  };
-  if constexpr (BULK) {
-    if (threadIdx.x == 0) {
-      mbar_init(&bar[0], 1);
-      mbar_init(&bar[1], 1);
-      mbar_init_fence();
-      mbar_arrive_expect(&bar[0], plane_bytes);  // planes zb-2 and zb-1
-      mbar_arrive_expect(&bar[1], plane_bytes);
-    }
-    __syncthreads();
-    issue(zb - CH);
-    issue(zb - CH + 1);
-    // prologue: planes zb-2 .. zb+1 into the ring, each slot refilled two planes ahead
-    for (int gz = zb - CH; gz < zb + CH; ++gz) {
-      const int late = fetch_plane(gz);
-      store_plane(slot_of(gz));
-      plane_barrier(late);
-      issue(gz + 2);
-    }
-  } else {
-    // prologue: planes zb-2 .. zb+1 into the ring, plane zb+2 into registers
-    for (int gz = zb - CH; gz < zb + CH; ++gz) {
-      load_plane(gz);
-      store_plane(slot_of(gz));
-    }
-    load_plane(zb + CH);
-  }
+  load_plane(zb + CH);
   const int gx = x0 + tx, gy = y0 + ty;
   const bool active = gx < b.n[0] && gy < b.n[1];
   const T id0 = cpar<T>(cp.invd[0], cp.invd_f[0]), id2 = cpar<T>(cp.invd[2], cp.invd_f[2]);
@@ -990,16 +856,9 @@ __global__ void __launch_bounds__(CX * CY, bulk_ctas<CentralFields<T, CONV, VISC
     for (int m = 0; m < 5; ++m) cw2[m] = r2 == 0 ? cpar<T>(cp.c2[0][m], cp.c2f[0][m]) : cpar<T>(cp.c2[1][m], cp.c2f[1][m]);
   }
   for (int gz = zb; gz < ze; ++gz) {
-    if constexpr (BULK) {
-      const int late = fetch_plane(gz + CH);  // copied during iteration gz - 2
-      store_plane(slot_of(gz + CH));
-      plane_barrier(late);
-      issue(gz + CH + 2);
-    } else {
-      store_plane(slot_of(gz + CH));  // plane gz+2, loaded during the previous iteration
-      __syncthreads();
-      if (gz + CH + 1 < ze + CH) load_plane(gz + CH + 1);
-    }
+    store_plane(slot_of(gz + CH));  // plane gz+2, loaded during the previous iteration
+    __syncthreads();
+    if (gz + CH + 1 < ze + CH) load_plane(gz + CH + 1);
     int pbase[2 * CH + 1];
 #pragma unroll
     for (int k = 0; k <= 2 * CH; ++k) pbase[k] = slot_of(gz + k - CH) * CPL;
@@ -1075,7 +934,7 @@ __global__ void __launch_bounds__(CX * CY, bulk_ctas<CentralFields<T, CONV, VISC
     T oh[5], ol[5];
     if (!first) {
 #pragma unroll
-      for (int v = (CONV || FUSE) ? 0 : 1; v < 5; ++v) r_load(b, v, gid, oh[v], ol[v]);
+      for (int v = FUSE ? 0 : 1; v < 5; ++v) r_load(b, v, gid, oh[v], ol[v]);
     }
     // the fused update's state and register, loaded before the derivative work hides them
     double fq[5], fo[5];
@@ -1091,94 +950,6 @@ __global__ void __launch_bounds__(CX * CY, bulk_ctas<CentralFields<T, CONV, VISC
     const T ID[3] = {id0, id1, id2};
     const T JD[3] = {jd0, jd1, jd2};
     const int UF[3] = {Fd::U0, Fd::U1, Fd::U2};
-    if (CONV == 1) {
-      // R_rho -= sum_j D_j m_j ; R_m_i -= D_i p + 1/2 sum_j [D_j(m_i u_j) + u_i D_j m_j + m_j D_j u_i]
-      // R_E -= sum_j [D_j(p u_j) + 1/2 (D_j(E u_j) + m_j D_j(E/rho) + (E/rho) D_j m_j)]
-      const int MF[3] = {Fd::M0, Fd::M1, Fd::M2};
-      T divm = L_(0.0);
-#pragma unroll
-      for (int j = 0; j < 3; ++j) divm += D1(MF[j], S[j], ID[j]);
-      racc[0] = -divm;
-      T Ec = F(Fd::E, 0) / F(Fd::RHO, 0);
-#pragma unroll
-      for (int i = 0; i < 3; ++i) {
-        T acc = D1(Fd::P, S[i], ID[i]);
-        T conv = L_(0.0), adv = L_(0.0);
-#pragma unroll
-        for (int j = 0; j < 3; ++j) {
-          const int s = S[j];
-          T pr = d1w<T>(F(MF[i], -2 * s) * F(UF[j], -2 * s), F(MF[i], -s) * F(UF[j], -s), F(MF[i], s) * F(UF[j], s),
-                        F(MF[i], 2 * s) * F(UF[j], 2 * s));
-          conv += pr * ID[j];
-          adv += F(MF[j], 0) * D1(UF[i], s, ID[j]);
-        }
-        acc += L_(0.5) * (conv + F(UF[i], 0) * divm + adv);
-        racc[1 + i] = -acc;
-      }
-      T e = L_(0.0);
-#pragma unroll
-      for (int j = 0; j < 3; ++j) {
-        const int s = S[j];
-        T dpu = d1w<T>(F(Fd::P, -2 * s) * F(UF[j], -2 * s), F(Fd::P, -s) * F(UF[j], -s), F(Fd::P, s) * F(UF[j], s),
-                       F(Fd::P, 2 * s) * F(UF[j], 2 * s));
-        T dEu = d1w<T>(F(Fd::E, -2 * s) * F(UF[j], -2 * s), F(Fd::E, -s) * F(UF[j], -s), F(Fd::E, s) * F(UF[j], s),
-                       F(Fd::E, 2 * s) * F(UF[j], 2 * s));
-        T dE = d1w<T>(F(Fd::E, -2 * s) / F(Fd::RHO, -2 * s), F(Fd::E, -s) / F(Fd::RHO, -s),
-                      F(Fd::E, s) / F(Fd::RHO, s), F(Fd::E, 2 * s) / F(Fd::RHO, 2 * s));
-        e += dpu * ID[j] + L_(0.5) * (dEu * ID[j] + F(MF[j], 0) * dE * ID[j]);
-      }
-      e += L_(0.5) * divm * Ec;
-      racc[4] = -e;
-    }
-    if (CONV == 2) {
-      // Kennedy-Gruber-Pirozzoli form (Fd::E holds H = (rhoE + p) / rho):
-      // R_rho = -1/2 sum_j [D_j m_j + rho du_j/dx_j + u_j D_j rho]
-      // R_m_i = -D_i p - 1/4 sum_j [D_j(u_i m_j) + rho D_j(u_i u_j) + u_i D_j m_j + u_j D_j m_i
-      //                             + m_i du_j/dx_j + m_j du_i/dx_j + u_i u_j D_j rho]
-      // R_E = -1/4 sum_j [D_j(H m_j) + rho D_j(H u_j) + H D_j m_j + u_j D_j(H rho) + m_j D_j H
-      //                   + H rho du_j/dx_j + H u_j D_j rho]
-      const int MF[3] = {Fd::M0, Fd::M1, Fd::M2};
-      auto DP = [&](int f, int g, int s, T inv) -> T {
-        return d1w<T>(F(f, -2 * s) * F(g, -2 * s), F(f, -s) * F(g, -s), F(f, s) * F(g, s), F(f, 2 * s) * F(g, 2 * s)) * inv;
-      };
-      const T rho0 = F(Fd::RHO, 0), H0 = F(Fd::E, 0);
-      T dm[3], drho[3], ujj = L_(0.0), divm = L_(0.0);
-#pragma unroll
-      for (int j = 0; j < 3; ++j) {
-        dm[j] = D1(MF[j], S[j], ID[j]);
-        drho[j] = D1(Fd::RHO, S[j], ID[j]);
-        ujj += D1(UF[j], S[j], ID[j]);
-        divm += dm[j];
-      }
-      T rc = divm + rho0 * ujj;
-#pragma unroll
-      for (int j = 0; j < 3; ++j) rc += F(UF[j], 0) * drho[j];
-      racc[0] = -L_(0.5) * rc;
-#pragma unroll
-      for (int i = 0; i < 3; ++i) {
-        const T ui = F(UF[i], 0), mi = F(MF[i], 0);
-        T acc = L_(0.0);
-#pragma unroll
-        for (int j = 0; j < 3; ++j) {
-          const int s = S[j];
-          const T uj = F(UF[j], 0);
-          acc += DP(UF[i], MF[j], s, ID[j]) + rho0 * DP(UF[i], UF[j], s, ID[j]) + ui * dm[j] +
-                 uj * D1(MF[i], s, ID[j]) + mi * D1(UF[j], s, ID[j]) + F(MF[j], 0) * D1(UF[i], s, ID[j]) +
-                 ui * uj * drho[j];
-        }
-        racc[1 + i] = -(D1(Fd::P, S[i], ID[i]) + L_(0.25) * acc);
-      }
-      T e = L_(0.0);
-#pragma unroll
-      for (int j = 0; j < 3; ++j) {
-        const int s = S[j];
-        const T uj = F(UF[j], 0);
-        e += DP(Fd::E, MF[j], s, ID[j]) + rho0 * DP(Fd::E, UF[j], s, ID[j]) + H0 * dm[j] +
-             uj * DP(Fd::E, Fd::RHO, s, ID[j]) + F(MF[j], 0) * D1(Fd::E, s, ID[j]) +
-             H0 * rho0 * D1(UF[j], s, ID[j]) + H0 * uj * drho[j];
-      }
-      racc[4] = -L_(0.25) * e;
-    }
     if (VISC) {
       T du[3][3], lap[3], dmu[3], dT[3], lapT = L_(0.0);
 #pragma unroll
@@ -1246,25 +1017,18 @@ __global__ void __launch_bounds__(CX * CY, bulk_ctas<CentralFields<T, CONV, VISC
         racc[4] -= w;
       }
     }
-    const int v0 = CONV ? 0 : 1;
+    const int v0 = 1;
     if constexpr (FUSE) {
       // a first (only) residual kernel starts from zero; otherwise from the partial residual
       unsigned nb = 0;
-      if (rf.kind == 0 && rf.a_zero) {  // uniform: the first low-storage stage, one FMA per variable
+      rk_modes(rf, [&](auto mode) {
 #pragma unroll
         for (int v = 0; v < 5; ++v) {
           float h = first ? racc[v] : oh[v], l = first ? 0.f : ol[v];
           if (!first && v >= v0) rp_final(racc[v], h, l);
-          nb += rk_point_a0(b, rf, v, gid, h, l, fq[v]);
+          nb += rk_point<decltype(mode)::value>(b, rf, v, gid, h, l, fq[v], fo[v]);
         }
-      } else {
-#pragma unroll
-        for (int v = 0; v < 5; ++v) {
-          float h = first ? racc[v] : oh[v], l = first ? 0.f : ol[v];
-          if (!first && v >= v0) rp_final(racc[v], h, l);
-          nb += rk_point_ff(b, rf, v, gid, h, l, fq[v], fo[v]);
-        }
-      }
+      });
       if (nb) atomicAdd(rf.bad, (unsigned long long)nb);
     } else if (first) {
 #pragma unroll
@@ -1275,13 +1039,6 @@ __global__ void __launch_bounds__(CX * CY, bulk_ctas<CentralFields<T, CONV, VISC
     }
     }  // active
     __syncthreads();  // the next iteration overwrites the slot of plane gz-2
-  }
-  if constexpr (BULK) {
-    // only a broken CTA can end with copies in flight: wait for them (bounded) before its
-    // shared memory is released
-#pragma unroll
-    for (int s2 = 0; s2 < 2; ++s2)
-      if (pend & (1u << s2)) mbar_wait_bounded(&bar[s2], (ppar >> s2) & 1u);
   }
 }
 

@@ -291,7 +291,7 @@ __global__ void __launch_bounds__(RT) k_resident_1d(const Resident1D* __restrict
             ff_flux_diff(fr, fl, invd_f, p, pe);
             const float hh = __fadd_rn(p, pe);
             const float ll = __fsub_rn(pe, __fsub_rn(hh, p));
-            const double x = dt_residual(hh, ll, dt_h, dt_l);  // as rk_point_ff
+            const double x = dt_residual(hh, ll, dt_h, dt_l);  // as rk_point
             if (rk.kind == 0) {
               ov = a_zero ? x : __fma_rn(A, ov, x);
               qv = __fma_rn(B, ov, qv);

@@ -90,7 +90,7 @@ int launch_wall(osb_ctx* c, Block& bl, int first, const RkFuse& rf) {
 template <typename T, int CONV, int VISC, bool FUSE, bool BULK>
 int launch_tile(osb_ctx* c, Block& bl, int first, const RkFuse& rf) {
   auto kern = k_central<T, CONV, VISC, FUSE, BULK>;
-  constexpr size_t smem = ct_smem<T, CONV, VISC, FUSE, BULK>();
+  constexpr size_t smem = ct_smem<T, CONV, VISC, BULK>();
   OSB_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const ColumnGrid g = column_grid(c, bl.k, kern, CTY, smem, sizeof(T) == 8 ? 0.9 : 1.4);
   timing_begin(c, FAM_CENTRAL);

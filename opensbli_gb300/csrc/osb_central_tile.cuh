@@ -27,9 +27,11 @@
 // constant viscosity), 615 and 1 030 before: 128^3 viscous 2.16 -> 1.38 ms, 64^3 Feiereisen 0.45 ->
 // 0.23 ms per launch.
 //
-// FP32, FUSE: half of the bytes are the update's (FP64 state and register); they come by cp.async a
-// plane ahead.  256^3 viscous + update 0.92 -> 0.84 ms per stage (240 bytes per point, 4.8 TB/s), 131 x
-// 97 x 110 0.109 -> 0.097, 64^3 Feiereisen + update 27 -> 24 us; KGP 128^3 0.168 -> 0.162 ms.
+// FP32, FUSE: half of the bytes are the update's (FP64 state and register), loaded at the start of a
+// plane's arithmetic; through shared memory a plane ahead (cp.async) they gained nothing (viscous) or
+// lost 20 % (KGP: one more CTA's worth of shared memory).  256^3 viscous + update 0.92 -> 0.82 ms per
+// stage (240 bytes per point, 4.9 TB/s), 131 x 97 x 110 0.109 -> 0.096, 64^3 Feiereisen + update 27 ->
+// 22 us, KGP 128^3 0.168 -> 0.133 ms.
 //
 // BULK (FP32 state only): the raw planes come in through the bulk-copy (TMA) engine instead --
 // one cp.async.bulk per staged row and variable into a two-slot raw buffer in shared memory,
@@ -55,22 +57,16 @@ struct CtFields {
   static constexpr int M = 3 + (VISC ? (VISC == 1 ? 2 : 1) : 0), EE = M + 3, HH = M + 4, P = M + 5;
   static constexpr int N = CONV ? (CONV == 2 && VISC ? M + 5 : M + 6) : M;
 };
-// FUSE: a thread's FP64 state and register and (CONV == 0) float-float residual of the next plane.
-template <int CONV, bool FUSE>
-struct CtUpdate {
-  static constexpr size_t bytes = FUSE ? (size_t)CTT * (10 * sizeof(double) + (CONV ? 0 : 10 * sizeof(float))) : 0;
-};
-template <typename T, int CONV, int VISC, bool FUSE, bool BULK>
+template <typename T, int CONV, int VISC, bool BULK>
 constexpr size_t ct_smem() {
   return sizeof(T) * ((size_t)CtFields<CONV, VISC>::N * CRING * CTPL + (VISC ? CSX * CTY + CX * CTSY : 0)) +
-         CtUpdate<CONV, FUSE>::bytes +
          (BULK ? CTRAW * sizeof(float) + 2 * sizeof(unsigned long long) : 0);
 }
 // CTAs per SM that the register allocation has to leave room for: what shared memory admits, at
 // most two (the update's FP64 values spill at the 80 registers of three).
-template <typename T, int CONV, int VISC, bool FUSE, bool BULK>
+template <typename T, int CONV, int VISC, bool BULK>
 constexpr int ct_ctas() {
-  return (228 * 1024) / (ct_smem<T, CONV, VISC, FUSE, BULK>() + 1024) >= 2 ? 2 : 1;
+  return (228 * 1024) / (ct_smem<T, CONV, VISC, BULK>() + 1024) >= 2 ? 2 : 1;
 }
 
 template <typename T>
@@ -85,21 +81,17 @@ __device__ __forceinline__ T fmat(T a, T b, T c) {
 }
 
 template <typename T, int CONV, int VISC, bool FUSE, bool BULK>
-__global__ void __launch_bounds__(CTT, ct_ctas<T, CONV, VISC, FUSE, BULK>())
+__global__ void __launch_bounds__(CTT, ct_ctas<T, CONV, VISC, BULK>())
     k_central(BlockK b, CentralParams cp, int first, int czc, RkFuse rf) {
   static_assert(!BULK || sizeof(T) == 4, "bulk staging: FP32 state");
   using Fd = CtFields<CONV, VISC>;
   constexpr int FS = CRING * CTPL;
   constexpr int V0 = CONV ? 0 : 1;  // first variable with a contribution
-  constexpr size_t UB = CtUpdate<CONV, FUSE>::bytes;
   extern __shared__ __align__(16) unsigned char osb_smem[];
   // BULK: the raw plane slots (rows 16-byte aligned), one mbarrier per slot, then the ring
   float* raw = reinterpret_cast<float*>(osb_smem);
   unsigned long long* bar = reinterpret_cast<unsigned long long*>(raw + CTRAW);
-  unsigned char* ring0 = osb_smem + (BULK ? CTRAW * sizeof(float) + 2 * sizeof(unsigned long long) : 0);
-  double (*upd)[CTT] = reinterpret_cast<double (*)[CTT]>(ring0);                    // FUSE: [10] q, rk
-  float (*res)[CTT] = reinterpret_cast<float (*)[CTT]>(ring0 + 10 * sizeof(double) * CTT);  // FUSE, CONV 0: [10] R
-  T* sm = reinterpret_cast<T*>(ring0 + UB);
+  T* sm = reinterpret_cast<T*>(osb_smem + (BULK ? CTRAW * sizeof(float) + 2 * sizeof(unsigned long long) : 0));
   T* Sx = sm + Fd::N * FS;       // [CTY][CSX]: D_y u_y + D_z u_z of the current plane
   T* Sy = Sx + CSX * CTY;        // [CTSY][CX]: D_x u_x + D_z u_z
   const int tx = threadIdx.x % CX, ty = threadIdx.x / CX;
@@ -275,26 +267,6 @@ __global__ void __launch_bounds__(CTT, ct_ctas<T, CONV, VISC, FUSE, BULK>())
     }
     load_plane(zb + CH);
   }
-  // FUSE: the point's FP64 state and register and partial residual of plane gz into this thread's
-  // slots, issued as soon as the previous plane's were used: the copies have a whole plane's
-  // arithmetic and barriers to arrive, and hold no registers meanwhile
-  auto fetch_update = [&](int gz) {
-    if constexpr (FUSE) {
-      if (active && gz < ze) {
-        const int id = lin(b, gx, gy, gz);
-#pragma unroll
-        for (int v = 0; v < 5; ++v) {
-          cp_async_el(&upd[v][threadIdx.x], b.q[v] + id);
-          if (!rf.a_zero) cp_async_el(&upd[5 + v][threadIdx.x], b.rk[v] + id);
-          if constexpr (CONV == 0) {
-            cp_async_el(&res[v][threadIdx.x], b.Rh[v] + id);
-            cp_async_el(&res[5 + v][threadIdx.x], b.Rl[v] + id);
-          }
-        }
-      }
-    }
-  };
-  fetch_update(zb);
   // this column's D_x u_x and D_y u_y of planes gz .. gz+2, and their sum of planes gz-2 .. gz+2
   T d00[3], d11[3], sz[5];
   if (VISC) {
@@ -324,10 +296,21 @@ __global__ void __launch_bounds__(CTT, ct_ctas<T, CONV, VISC, FUSE, BULK>())
 #pragma unroll
     for (int k = 0; k <= 2 * CH; ++k) pb[k] = slot_of(gz + k - CH) * CTPL;
     const int gid = lin(b, gx, gy, gz);
-    T oh[5], ol[5];  // the partial residual (FUSE: from `res`)
-    if (!FUSE && active && !first) {
+    // the partial residual, and the fused update's state and register, before the arithmetic
+    T oh[5], ol[5];
+    if (active && !first) {
 #pragma unroll
-      for (int v = V0; v < 5; ++v) r_load(b, v, gid, oh[v], ol[v]);
+      for (int v = FUSE ? 0 : V0; v < 5; ++v) r_load(b, v, gid, oh[v], ol[v]);
+    }
+    double fq[5], fo[5];
+    if constexpr (FUSE) {
+      if (active) {
+#pragma unroll
+        for (int v = 0; v < 5; ++v) {
+          fq[v] = b.q[v][gid];
+          fo[v] = rf.a_zero ? 0.0 : b.rk[v][gid];
+        }
+      }
     }
     T du[3][3];
     if (VISC) {
@@ -522,7 +505,6 @@ __global__ void __launch_bounds__(CTT, ct_ctas<T, CONV, VISC, FUSE, BULK>())
       if constexpr (FUSE) {
         // the central scheme's only residual kernel starts from zero, the viscous terms of a
         // shock-capturing block from the sweeps' partial residual
-        cp_async_wait_all();
         unsigned nb = 0;
         rk_modes(rf, [&](auto mode) {
           constexpr int MODE = decltype(mode)::value;
@@ -530,14 +512,13 @@ __global__ void __launch_bounds__(CTT, ct_ctas<T, CONV, VISC, FUSE, BULK>())
           for (int v = 0; v < 5; ++v) {
             float h = racc[v], l = 0.f;
             if constexpr (CONV == 0) {
-              h = res[v][threadIdx.x];
-              l = res[5 + v][threadIdx.x];
+              h = oh[v];
+              l = ol[v];
               if (v >= V0) rp_final(racc[v], h, l);
             }
-            nb += rk_point<MODE>(b, rf, v, gid, h, l, upd[v][threadIdx.x], MODE == 0 ? 0.0 : upd[5 + v][threadIdx.x]);
+            nb += rk_point<MODE>(b, rf, v, gid, h, l, fq[v], fo[v]);
           }
         });
-        fetch_update(gz + 1);
         if (nb) atomicAdd(rf.bad, (unsigned long long)nb);
       } else if (first) {
 #pragma unroll

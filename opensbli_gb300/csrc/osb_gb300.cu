@@ -110,10 +110,34 @@ __global__ void k_q2qf(BlockK b, int nv) {
 // Halo arrays a boundary kernel writes: the FP64 state, the FP32 state, or both.
 enum { BC_Q = 1, BC_QF = 2, BC_BOTH = 3 };
 
+// All variables of a point from si to di (FP64 and / or FP32 state): every load before the first store.
+__device__ __forceinline__ void copy_point(double* const* dq, const double* const* sq, float* const* dqf,
+                                           const float* const* sqf, int nv, int di, int si, int fields) {
+  if (fields & BC_Q) {
+    double x[5];
+#pragma unroll
+    for (int v = 0; v < 5; ++v)
+      if (v < nv) x[v] = sq[v][si];
+#pragma unroll
+    for (int v = 0; v < 5; ++v)
+      if (v < nv) dq[v][di] = x[v];
+  }
+  if ((fields & BC_QF) && dqf[0]) {
+    float x[5];
+#pragma unroll
+    for (int v = 0; v < 5; ++v)
+      if (v < nv) x[v] = sqf[v][si];
+#pragma unroll
+    for (int v = 0; v < 5; ++v)
+      if (v < nv) dqf[v][di] = x[v];
+  }
+}
+
 // Periodic exchange of both faces of direction d (ExchangeSelf, periodic.py:53-71):
 // side 0 copies [0, depth) to [N, N+depth), side 1 copies [N-depth, N) to [-depth, 0); the
 // transverse ranges include -depth..N+depth of the other used directions (corners).
-// blockIdx.y = 2 * variable + side; 32-bit index arithmetic.
+// blockIdx.y = side; a thread moves all variables of a point (one index calculation, its loads in
+// flight together); 32-bit index arithmetic.
 __global__ void k_periodic(BlockK b, int nv, int d, int depth0, int depth1, int fields) {
   const int dmax = max(depth0, depth1);
   int ext[3], lo[3];
@@ -127,7 +151,7 @@ __global__ void k_periodic(BlockK b, int nv, int d, int depth0, int depth1, int 
     }
   }
   ext[d] = dmax;
-  const int side = blockIdx.y & 1, v = blockIdx.y >> 1;
+  const int side = blockIdx.y;
   const int depth = side == 0 ? depth0 : depth1;
   const int N = b.n[d];
   const int per = ext[0] * ext[1] * ext[2];
@@ -154,8 +178,7 @@ __global__ void k_periodic(BlockK b, int nv, int d, int depth0, int depth1, int 
       dst[d] = -depth + c[d];
     }
     const int di = lin(b, dst[0], dst[1], dst[2]), si = lin(b, src[0], src[1], src[2]);
-    if (fields & BC_Q) b.q[v][di] = b.q[v][si];
-    if ((fields & BC_QF) && b.qf[0]) b.qf[v][di] = b.qf[v][si];
+    copy_point(b.q, b.q, b.qf, b.qf, nv, di, si, fields);
   }
 }
 
@@ -200,16 +223,7 @@ __global__ void k_periodic_shell(BlockK b, int nv, int D, int fields) {
     const int sy = y < 0 ? y + n1 : (y >= n1 ? y - n1 : y);
     const int sz = z < 0 ? z + n2 : (z >= n2 ? z - n2 : z);
     const int di = lin(b, x, y, z), si = lin(b, sx, sy, sz);
-    if (fields & BC_Q) {
-      double vq[5];
-      for (int v = 0; v < nv; ++v) vq[v] = b.q[v][si];
-      for (int v = 0; v < nv; ++v) b.q[v][di] = vq[v];
-    }
-    if ((fields & BC_QF) && b.qf[0]) {
-      float vf[5];
-      for (int v = 0; v < nv; ++v) vf[v] = b.qf[v][si];
-      for (int v = 0; v < nv; ++v) b.qf[v][di] = vf[v];
-    }
+    copy_point(b.q, b.q, b.qf, b.qf, nv, di, si, fields);
   }
 }
 
@@ -414,25 +428,43 @@ __device__ void wall_point(A* const* q, int nd, int w, int o, int depth, A gm, A
   using O = WOp<A>;
   const int nv = nd + 2;
   const A g1 = O::add(gm, A(-1));
+  // the layers inside, before the first store: their loads are in flight together
+  A in[5][4], Ea = A(0);  // density and momentum of the points 1 .. depth inside, energy of the first
+#pragma unroll
+  for (int k = 0; k < 5; ++k)
+    if (k < depth || k == 0)
+#pragma unroll
+      for (int v = 0; v < 4; ++v)
+        if (v <= nd) in[k][v] = q[v][w + (k + 1) * o];
+  Ea = q[nv - 1][w + o];
+  const A rw = q[0][w];
   for (int i = 0; i < nd; ++i) q[1 + i][w] = A(0);
-  q[nv - 1][w] = O::div(O::mul(Tw, q[0][w]), O::mul(O::mul(gm, M2), g1));
-  const A pw = O::mul(g1, q[nv - 1][w]);
-  const int a = w + o;
+  const A Ew = O::div(O::mul(Tw, rw), O::mul(O::mul(gm, M2), g1));
+  q[nv - 1][w] = Ew;
+  const A pw = O::mul(g1, Ew);
   A ke = A(0);
-  for (int i = 0; i < nd; ++i) ke = O::add(ke, O::mul(A(0.5), O::mul(q[1 + i][a], q[1 + i][a])));
-  const A ra = q[0][a];
-  const A Ta = O::div(O::mul(O::mul(O::mul(M2, g1), O::add(q[nv - 1][a], -O::div(ke, ra))), gm), ra);
-  for (int k = 1; k <= depth; ++k) {
-    const int in = w + k * o, h = w - k * o;
+#pragma unroll
+  for (int i = 0; i < 3; ++i)
+    if (i < nd) ke = O::add(ke, O::mul(A(0.5), O::mul(in[0][1 + i], in[0][1 + i])));
+  const A ra = in[0][0];
+  const A Ta = O::div(O::mul(O::mul(O::mul(M2, g1), O::add(Ea, -O::div(ke, ra))), gm), ra);
+#pragma unroll
+  for (int k = 1; k <= 5; ++k) {
+    if (k > depth) break;
+    const int h = w - k * o;
     A u[3], u2 = A(0);
-    for (int i = 0; i < nd; ++i) {
-      u[i] = O::div(q[1 + i][in], q[0][in]);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      if (i >= nd) continue;
+      u[i] = O::div(in[k - 1][1 + i], in[k - 1][0]);
       u2 = O::add(u2, O::mul(u[i], u[i]));
     }
     const A Tk = O::add(O::mul(A(-k), Ta), O::mul(A(k + 1), Tw));
     const A rk = O::div(O::mul(O::mul(M2, gm), pw), Tk);
     q[0][h] = rk;
-    for (int i = 0; i < nd; ++i) q[1 + i][h] = -O::mul(rk, u[i]);
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+      if (i < nd) q[1 + i][h] = -O::mul(rk, u[i]);
     q[nv - 1][h] = O::add(O::div(pw, g1), O::mul(O::mul(A(0.5), u2), rk));
   }
 }
@@ -533,7 +565,7 @@ __global__ void k_dirichlet(BlockK b, int nv, int d, int side, int depth, int ha
 // finds its face from the faces' starting offsets.
 constexpr int kIfMax = 24;
 struct IfFace {
-  long begin;                  // first element of this face in the launch's index space
+  int begin;                   // first point of this face in the launch's index space
   int d, side, sside, flip, depth, nv;
   int ext[3], lo[3];           // copied box: extents and lower corner (transverse), layers along d
   int dn[3], dst_st[3], dst_off0;
@@ -545,21 +577,20 @@ struct IfFace {
 };
 struct IfBatch {
   int nfaces;
-  long total;
+  int total;  // points of all faces
   IfFace f[kIfMax];
 };
 
 __global__ void k_interface(const __grid_constant__ IfBatch batch, int fields) {
-  for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < batch.total; t += (long)gridDim.x * blockDim.x) {
+  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < batch.total; t += gridDim.x * blockDim.x) {
     int i = 0;
     while (i + 1 < batch.nfaces && batch.f[i + 1].begin <= t) ++i;
     const IfFace& F = batch.f[i];
-    long r = t - F.begin;
+    int r = t - F.begin;
     int c[3];
-    c[0] = (int)(r % F.ext[0]); r /= F.ext[0];
-    c[1] = (int)(r % F.ext[1]); r /= F.ext[1];
-    c[2] = (int)(r % F.ext[2]);
-    const int v = (int)(r / F.ext[2]);
+    c[0] = r % F.ext[0]; r /= F.ext[0];
+    c[1] = r % F.ext[1];
+    c[2] = r / F.ext[1];
     int di[3], si[3];
     for (int e = 0; e < 3; ++e) di[e] = si[e] = c[e] + F.lo[e];
     di[F.d] = F.side == 0 ? -F.depth + c[F.d] : F.dn[F.d] + c[F.d];
@@ -567,8 +598,7 @@ __global__ void k_interface(const __grid_constant__ IfBatch batch, int fields) {
     si[F.d] = F.sside == 1 ? F.sn[F.d] - F.depth + sl : sl;
     const int a = F.dst_off0 + di[0] * F.dst_st[0] + di[1] * F.dst_st[1] + di[2] * F.dst_st[2];
     const int bs = F.src_off0 + si[0] * F.src_st[0] + si[1] * F.src_st[1] + si[2] * F.src_st[2];
-    if (fields & BC_Q) F.dq[v][a] = F.sq[v][bs];
-    if ((fields & BC_QF) && F.dqf[0]) F.dqf[v][a] = F.sqf[v][bs];
+    copy_point(F.dq, F.sq, F.dqf, F.sqf, F.nv, a, bs, fields);
   }
 }
 
@@ -842,7 +872,7 @@ int apply_interfaces(osb_ctx* c, int full, int fields) {
         F.flip = f.flip;
         F.depth = depth;
         F.nv = nv;
-        long total = nv;
+        long total = 1;
         for (int e = 0; e < 3; ++e) {
           if (e < bl.d.ndim && e != d) {
             F.lo[e] = full ? -depth : 0;
@@ -866,8 +896,8 @@ int apply_interfaces(osb_ctx* c, int full, int fields) {
           F.dqf[v] = v < nv ? bl.k.qf[v] : nullptr;
           F.sqf[v] = v < nv ? nb.k.qf[v] : nullptr;
         }
-        batch.total += total;
-        if (++batch.nfaces == kIfMax) flush();
+        batch.total += (int)total;
+        if (++batch.nfaces == kIfMax || batch.total > (1 << 30)) flush();
       }
   }
   flush();
@@ -920,8 +950,7 @@ int apply_block_bc(osb_ctx* c, Block& bl, size_t ib, int fields) {
         if (e != d) tr *= bl.k.n[e] + 2 * std::max(dep0, dep1);
       long per = (long)std::max(dep0, dep1) * tr;
       timing_begin(c, FAM_BC);
-      k_periodic<<<dim3(std::max(1, grid_for(c, per, 256) / (2 * nv) + 1), 2 * nv), 256, 0, c->stream>>>(
-          bl.k, nv, d, dep0, dep1, fields);
+      k_periodic<<<dim3(grid_for(c, per, 256), 2), 256, 0, c->stream>>>(bl.k, nv, d, dep0, dep1, fields);
       timing_end(c);
       c->launches++;
       continue;

@@ -519,7 +519,8 @@ __global__ void __launch_bounds__(SWEEP_THREADS, sizeof(T) == 4 ? 3 : 1)
 // osb_set_variant.  Row pitches are odd, so the 32 lanes (rows) of a warp hit distinct banks.
 constexpr int XCH = 4, XRING = 2, XCOLS = XCH * XRING, XPITCH = XCOLS + 1, XOUT = 8, XOPITCH = XOUT + 1;
 // FP32: six CTAs of two warps per SM, 168 registers (256^3 TENO5: 0.61 ms; 0.76 with eight CTAs at
-// 128; 0.86 before the packed flux).
+// 128; 0.86 before the packed flux).  Curvilinear: four CTAs, 255 registers (4-block case 2.8 ms a
+// step; 4.8 with six).
 constexpr int XWARPS = 2;
 
 template <typename T, int NF, int NO>
@@ -530,7 +531,7 @@ struct XTile {
 };
 
 template <typename T, int ND, int SCH, int AVG, bool CURV, int FLX = 0>
-__global__ void __launch_bounds__(32 * XWARPS, sizeof(T) == 4 ? 6 : 1) k_flux_x(BlockK b, SchemeParams spd, int first, int xseg,
+__global__ void __launch_bounds__(32 * XWARPS, sizeof(T) == 4 ? (CURV ? 4 : 6) : 1) k_flux_x(BlockK b, SchemeParams spd, int first, int xseg,
                                                          const int* __restrict__ xrows) {
   constexpr int NV = ND + 2;
   constexpr int NF = SweepFields<ND, CURV>::N;

@@ -87,9 +87,12 @@ int launch_wall(osb_ctx* c, Block& bl, int first, const RkFuse& rf) {
   return OSB_OK;
 }
 
-template <typename T, int CONV, int VISC, bool FUSE, bool BULK>
+template <typename T, int CONV, int VISC, bool FUSE, bool BULK, bool WRAP = false>
 int launch_tile(osb_ctx* c, Block& bl, int first, const RkFuse& rf) {
-  auto kern = k_central<T, CONV, VISC, FUSE, BULK>;
+  if constexpr (CONV != 0 && !BULK && !WRAP) {
+    if (bl.k.wrap) return launch_tile<T, CONV, VISC, FUSE, BULK, true>(c, bl, first, rf);
+  }
+  auto kern = k_central<T, CONV, VISC, FUSE, BULK, WRAP>;
   constexpr size_t smem = ct_smem<T, CONV, VISC, BULK>();
   OSB_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const ColumnGrid g = column_grid(c, bl.k, kern, CTY, smem, sizeof(T) == 8 ? 0.9 : 1.4);

@@ -1021,16 +1021,20 @@ int apply_block_bc(osb_ctx* c, Block& bl, size_t ib, int fields) {
 // Boundary conditions of all blocks: interface faces (interior of the face), then each
 // block's own faces (apply_block_bc), then the interface faces again with their transverse
 // halos, which the neighbour has filled by then.
-int apply_bc(osb_ctx* c, int fields = BC_BOTH) {
+// With `which` the call covers only the blocks read in place (WRAPPED) or only the others (NOT_WRAPPED).
+enum BcBlocks { ALL_BLOCKS, NOT_WRAPPED, WRAPPED };
+int apply_bc(osb_ctx* c, int fields = BC_BOTH, BcBlocks which = ALL_BLOCKS) {
   bool any_iface = false;
   for (auto& bl : c->blocks)
     for (int d = 0; d < bl.d.ndim; ++d)
       any_iface = any_iface || bl.d.bc[d][0] == OSB_BC_INTERFACE || bl.d.bc[d][1] == OSB_BC_INTERFACE;
+  if (which == WRAPPED) any_iface = false;  // a wrapped block has no interface
   if (any_iface) {
     int rc = apply_interfaces(c, 0, fields);
     if (rc) return rc;
   }
   for (size_t ib = 0; ib < c->blocks.size(); ++ib) {
+    if (which != ALL_BLOCKS && (c->blocks[ib].k.wrap != 0) != (which == WRAPPED)) continue;
     int rc = apply_block_bc(c, c->blocks[ib], ib, fields);
     if (rc) return rc;
   }
@@ -1079,7 +1083,7 @@ int stage(osb_ctx* c, int s, double dt, bool bc = true) {
     batch_set_parity(c, c->qf_parity ^ 1);
     // between stages the FP32 kernels read only the FP32 state; the FP64 halos are refreshed
     // when a call returns (osb_step / osb_stage)
-    return bc ? apply_bc(c, BC_QF) : OSB_OK;
+    return bc ? apply_bc(c, BC_QF, NOT_WRAPPED) : OSB_OK;
   }
   for (auto& bl : c->blocks) {
     int rc = residual(c, bl);
@@ -1092,7 +1096,7 @@ int stage(osb_ctx* c, int s, double dt, bool bc = true) {
     timing_end(c);
     c->launches++;
   }
-  return bc ? apply_bc(c) : OSB_OK;
+  return bc ? apply_bc(c, BC_BOTH, NOT_WRAPPED) : OSB_OK;
 }
 
 bool any_filter(const osb_ctx* c, int kind) {
@@ -1123,7 +1127,7 @@ int one_step(osb_ctx* c, double dt) {
     }
     return OSB_OK;
   }
-  int rc = apply_bc(c, c->prec == OSB_PREC_FP32_RESIDUAL ? BC_QF : BC_BOTH);
+  int rc = apply_bc(c, c->prec == OSB_PREC_FP32_RESIDUAL ? BC_QF : BC_BOTH, NOT_WRAPPED);
   if (rc) return rc;
   if (c->rk_kind == OSB_RK_SBLI3) {
     for (auto& bl : c->blocks) {
@@ -1791,11 +1795,29 @@ int osb_apply_bc(osb_ctx* c) {
 
 namespace {
 
-// Halos that a caller observes when a call of the FP32-residual path returns.
+// Halos that a caller observes when osb_step returns: all of the FP32-residual path's (between stages
+// it keeps the FP32 state's alone), on the FP64 path those of the blocks read in place.
 int observer_halos(osb_ctx* c, bool batch) {
+  if (c->prec == OSB_PREC_FP64) return apply_bc(c, BC_BOTH, WRAPPED);
   if (batch && batch_halo(c)) return OSB_OK;
   return apply_bc(c, batch ? BC_BOTH : BC_Q);
 }
+
+}  // namespace
+
+namespace {
+
+// Marks the blocks that osb_step reads in place while it queues work.
+struct WrapScope {
+  osb_ctx* c;
+  explicit WrapScope(osb_ctx* ctx) : c(ctx) {
+    const bool bulk = c->prec == OSB_PREC_FP32_RESIDUAL && c->central_bulk;  // bulk copies read rows as they lie
+    for (auto& bl : c->blocks) bl.k.wrap = !bulk && bl.can_wrap() ? 1 : 0;
+  }
+  ~WrapScope() {
+    for (auto& bl : c->blocks) bl.k.wrap = 0;
+  }
+};
 
 }  // namespace
 
@@ -1812,6 +1834,7 @@ int osb_step(osb_ctx* c, double dt, int nsteps) {
     OSB_CK(cudaGetLastError());
     return OSB_OK;
   }
+  const WrapScope wrap(c);
   const bool batch = use_batch(c);
   if (batch && !c->batch.ready) {
     int rc = batch_build(c);  // allocates: never inside a capture
@@ -1824,7 +1847,7 @@ int osb_step(osb_ctx* c, double dt, int nsteps) {
       int rc = one_step(c, dt);
       if (rc) return rc;
     }
-    if (c->prec == OSB_PREC_FP32_RESIDUAL) {
+    if (nsteps > 0 || c->prec == OSB_PREC_FP32_RESIDUAL) {
       int rc = observer_halos(c, batch);
       if (rc) return rc;
     }
@@ -1890,6 +1913,11 @@ int osb_step(osb_ctx* c, double dt, int nsteps) {
   for (int it = 0; it < nsteps; ++it) {
     OSB_CK(cudaGraphLaunch(c->gexec, c->stream));
     c->launches += c->g_kernels;
+  }
+  if (nsteps > 0) {
+    int rc = observer_halos(c, batch);
+    if (rc) return rc;
+    OSB_CK(cudaGetLastError());
   }
   return OSB_OK;
 }

@@ -19,6 +19,7 @@ struct BlockK {
   int ndim;
   int st[3];       // linear strides of the OPS-layout arrays (32-bit: 64-bit integer multiplies
   int off0;        // would compete for the FP64 pipe); linear index of point (0,0,0)
+  int wrap;        // host flag: the central kernel reads the periodic images in place (k_central WRAP)
   long alloc;      // allocated points per array (< 2^31, checked at osb_block_add)
   double* q[5];
   double* rk[5];

@@ -178,10 +178,44 @@ static __device__ const double teno5_rows[8][4] = {
     OSB_TENO5_ROW(11.0, 8.0, 1.0, 20.0)};
 #undef OSB_TENO5_ROW
 
-// WENO5-Z / WENO5-JS with the IEEE divisions of the generated form, for values beyond the range of
-// the common denominator.
+template <int ND, int SCH>
+__host__ __device__ constexpr bool generated_order() {
+  return ND <= 2 && (SCH == SCH_TENO5 || SCH == SCH_TENO6);
+}
+
+// Fifth-order reconstruction in the generated order with IEEE divisions, FP64.  It serves
+//   - values beyond the range of recon5_f64's common denominator,
+//   - TENO5 on 1D and 2D blocks (generated_order; TENO6 keeps it too).  A front in exactly uniform gas is symmetric
+//     at first, so the outer indicators of a five-point window tie while the middle one is zero to
+//     rounding: tau is then the rounding of b0 - b2, and whether it is exactly zero decides if TENO5
+//     keeps the outer stencils.  Another order of the same operations moves a shock tube by 1e-7
+//     and a shear layer by 1e-5 of their size within ten steps (the WENO weights: below 1e-14).  3D
+//     blocks, with smooth fields in all directions, take recon5_f64 (a step of the 128^3 TENO5 vortex in
+//     the generated order 63 ms, with it 17).
 template <int SCH>
-static __device__ __noinline__ double weno5_wide(double fm2, double fm1, double f0, double fp1, double fp2, double eps) {
+__device__ __forceinline__ double recon5_ieee(double fm2, double fm1, double f0, double fp1, double fp2, double eps,
+                                              double ct) {
+  if (SCH == SCH_TENO5) {
+    const double s0 = fm1 - fp1, c0 = fm1 - 2.0 * f0 + fp1;
+    const double s1 = 3.0 * f0 - 4.0 * fp1 + fp2, c1 = f0 - 2.0 * fp1 + fp2;
+    const double s2 = fm2 - 4.0 * fm1 + 3.0 * f0, c2 = fm2 - 2.0 * fm1 + f0;
+    const double b0 = 0.25 * s0 * s0 + (13.0 / 12.0) * c0 * c0;
+    const double b1 = 0.25 * s1 * s1 + (13.0 / 12.0) * c1 * c1;
+    const double b2 = 0.25 * s2 * s2 + (13.0 / 12.0) * c2 * c2;
+    const double tau = fabs(b0 - b2);
+    const double t0 = 1.0 + tau / (eps + b0), t1 = 1.0 + tau / (eps + b1), t2 = 1.0 + tau / (eps + b2);
+    const double a0 = t0 * t0 * t0 * t0 * t0 * t0;
+    const double a1 = t1 * t1 * t1 * t1 * t1 * t1;
+    const double a2 = t2 * t2 * t2 * t2 * t2 * t2;
+    const double inv = 1.0 / (a0 + a1 + a2);
+    const double w0 = (11.0 / 20.0) * ((a0 * inv < ct) ? 0.0 : 1.0), w1 = (4.0 / 10.0) * ((a1 * inv < ct) ? 0.0 : 1.0),
+                 w2 = (1.0 / 20.0) * ((a2 * inv < ct) ? 0.0 : 1.0);
+    const double iw = 1.0 / (w0 + w1 + w2);
+    const double e0 = -(1.0 / 6.0) * fm1 + (5.0 / 6.0) * f0 + (2.0 / 6.0) * fp1;
+    const double e1 = (2.0 / 6.0) * f0 + (5.0 / 6.0) * fp1 - (1.0 / 6.0) * fp2;
+    const double e2 = (2.0 / 6.0) * fm2 - (7.0 / 6.0) * fm1 + (11.0 / 6.0) * f0;
+    return (w0 * e0 + w1 * e1 + w2 * e2) * iw;
+  }
   const double c0 = f0 - 2.0 * fp1 + fp2, s0 = 3.0 * f0 - 4.0 * fp1 + fp2;
   const double c1 = fm1 - 2.0 * f0 + fp1, s1 = fm1 - fp1;
   const double c2 = fm2 - 2.0 * fm1 + f0, s2 = fm2 - 4.0 * fm1 + 3.0 * f0;
@@ -205,6 +239,10 @@ static __device__ __noinline__ double weno5_wide(double fm2, double fm1, double 
   const double e1 = -(1.0 / 6.0) * fm1 + (5.0 / 6.0) * f0 + (1.0 / 3.0) * fp1;
   const double e2 = (1.0 / 3.0) * fm2 - (7.0 / 6.0) * fm1 + (11.0 / 6.0) * f0;
   return (a0 * inv) * e0 + (a1 * inv) * e1 + (a2 * inv) * e2;
+}
+template <int SCH>
+static __device__ __noinline__ double recon5_wide(double fm2, double fm1, double f0, double fp1, double fp2, double eps) {
+  return recon5_ieee<SCH>(fm2, fm1, f0, fp1, fp2, eps, 0.0);
 }
 
 // The epsilons of a scheme in the units of the reconstructed values: a caller that reconstructs
@@ -262,7 +300,7 @@ __device__ __forceinline__ double recon5_f64(double fm2, double fm1, double f0, 
   // Nn, D and 1 / D stay inside FP64's range for indicators between 1e-47 and 1e43; beyond
   // (values above 1e21) the generated form takes over
   const int de = (__double2hiint(D) >> 20) & 0x7ff;
-  if (de < 64 || de > 1903) return weno5_wide<SCH>(fm2, fm1, f0, fp1, fp2, e.eps);
+  if (de < 64 || de > 1903) return recon5_wide<SCH>(fm2, fm1, f0, fp1, fp2, e.eps);
   return __fma_rn(Nn, rcp_newton(D), f0);
 }
 
@@ -412,13 +450,20 @@ __device__ __forceinline__ T recon6(T fm2, T fm1, T f0, T fp1, T fp2, T fp3, con
 }
 
 // Reconstruction of one characteristic wave at i+1/2 from the positive and negative split
-// fluxes at points i-2..i+3.
-template <typename T, int SCH>
+// fluxes at points i-2..i+3 (GEN: FP64 in the generated order).
+template <typename T, int SCH, bool GEN = false>
 __device__ __forceinline__ T recon_wave(const T (&fp)[6], const T (&fm)[6], const SP<T>& sp) {
-  if (SCH == SCH_TENO6)
+  if constexpr (SCH == SCH_TENO6) {
     return recon6<T, 1>(fp[0], fp[1], fp[2], fp[3], fp[4], fp[5], sp) +
            recon6<T, -1>(fm[0], fm[1], fm[2], fm[3], fm[4], fm[5], sp);
-  return recon5<T, SCH>(fp[0], fp[1], fp[2], fp[3], fp[4], sp) + recon5<T, SCH>(fm[5], fm[4], fm[3], fm[2], fm[1], sp);
+  } else if constexpr (GEN && sizeof(T) == 8) {
+    const double eps = recon_eps<SCH>(sp.teno_eps, 1.0).eps;
+    return recon5_ieee<SCH>(fp[0], fp[1], fp[2], fp[3], fp[4], eps, sp.teno_ct) +
+           recon5_ieee<SCH>(fm[5], fm[4], fm[3], fm[2], fm[1], eps, sp.teno_ct);
+  } else {
+    return recon5<T, SCH>(fp[0], fp[1], fp[2], fp[3], fp[4], sp) +
+           recon5<T, SCH>(fm[5], fm[4], fm[3], fm[2], fm[1], sp);
+  }
 }
 
 // Point data carried through a sweep: conserved state in the local frame plus primitives.
@@ -465,6 +510,20 @@ struct Pt<double, ND> {
 };
 template <typename T, int ND>
 __device__ __forceinline__ void make_pt(Pt<double, ND>& s, double gm) {
+  if constexpr (ND <= 2) {  // the generated order (recon5_ieee)
+    const double rho = s.q[0], ir = 1.0 / rho;
+    double ke = 0.0;
+#pragma unroll
+    for (int i = 0; i < ND; ++i) {
+      s.u[i] = s.q[1 + i] * ir;
+      ke += s.u[i] * s.u[i];
+    }
+    s.p = (gm - 1.0) * (s.q[ND + 1] - 0.5 * rho * ke);
+    s.a = sqrt(gm * s.p * ir);
+    s.s = sqrt(rho);
+    s.H = (s.q[ND + 1] + s.p) * ir;
+    return;
+  }
   const double ir = rcp_newton(s.q[0]);
   double ke2 = 0.0;
 #pragma unroll
@@ -520,18 +579,28 @@ __device__ __forceinline__ void face_average_f64(const Pt<double, ND>& L, const 
 // -(gama - 1) / a^2 p (u_n' - u_n) in the entropy row.  A
 // row's constant factor commutes with the reconstruction (its epsilon is scaled instead, ReconEps),
 // so neither it nor the 1/2 of the flux splitting is applied to the twelve values of a wave, and
-// 1D, 2D and 3D share the form: their rows differ by that factor alone.
+// 1D, 2D and 3D share the form: their rows differ by that factor alone.  (generated_order: not here.)
 //
 // One interface of a 3D TENO5 block takes about 360 FP64 instructions here, against the 2 300 that
 // the generated order costs: a step of the 128^3 TENO5 vortex took 63.4 ms before and 19.2 ms with
 // it (6.8 of them in the central and update kernels), the 457 x 255 WENO5-Z shock reflection 2.21
 // and 1.12 ms, at the same error against plain 64-bit arithmetic (2e-16; TENO5 decides alike).
-template <int ND, int SCH, int AVG>
-__device__ __forceinline__ void char_flux_f64(const Pt<double, ND> (&w)[6], const SP<double>& sp, double (&fh)[ND + 2]) {
+// A register window as the window that char_flux_f64 reads.
+template <int ND>
+struct WindowF64 {
+  const Pt<double, ND> (&w)[6];
+  __device__ __forceinline__ const Pt<double, ND>& side(int m) const { return w[m]; }
+  __device__ __forceinline__ double q(int m, int v) const { return w[m].q[v]; }
+  __device__ __forceinline__ double un(int m) const { return w[m].u[0]; }
+  __device__ __forceinline__ double p(int m) const { return w[m].p; }
+};
+
+// A(m) gives point m of the window: the six of a register window, or of a tile in shared memory.
+template <int ND, int SCH, int AVG, typename Acc>
+__device__ __forceinline__ void char_flux_f64(const Acc& A, const SP<double>& sp, double (&fh)[ND + 2]) {
   constexpr int NV = ND + 2, E = ND + 1;
   const double g1 = sp.g1;
-  const Pt<double, ND>& L = w[2];
-  const Pt<double, ND>& R = w[3];
+  const Pt<double, ND> L = A.side(2), R = A.side(3);
   double u[ND], a, ia, rho2, ke;
   face_average_f64<ND, AVG>(L, R, g1, u, a, ia, rho2, ke);
   const double hk = 0.5 * ke, gi = g1 * ia, g = gi * ia;
@@ -541,12 +610,12 @@ __device__ __forceinline__ void char_flux_f64(const Pt<double, ND> (&w)[6], cons
   double P[6], D[6], W[6];
 #pragma unroll
   for (int m = 0; m < 6; ++m) {
-    double x = w[m].q[E];
+    double x = A.q(m, E);
 #pragma unroll
-    for (int i = 0; i < ND; ++i) x = __fma_rn(-u[i], w[m].q[1 + i], x);
-    P[m] = __fma_rn(hk, w[m].q[0], x);
-    D[m] = __fma_rn(-u[0], w[m].q[0], w[m].q[1]);
-    W[m] = w[m].p * (w[m].u[0] - u[0]);
+    for (int i = 0; i < ND; ++i) x = __fma_rn(-u[i], A.q(m, 1 + i), x);
+    P[m] = __fma_rn(hk, A.q(m, 0), x);
+    D[m] = __fma_rn(-u[0], A.q(m, 0), A.q(m, 1));
+    W[m] = A.p(m) * (A.un(m) - u[0]);
   }
   // reconstruction of one wave from its split fluxes, twice a scale times the generated ones: s2 is
   // that factor squared; TENO6, whose side +1 indicator is not homogeneous, takes them unscaled
@@ -571,9 +640,9 @@ __device__ __forceinline__ void char_flux_f64(const Pt<double, ND> (&w)[6], cons
   // entropy wave
 #pragma unroll
   for (int m = 0; m < 6; ++m) {
-    const double c = __fma_rn(-g, P[m], w[m].q[0]), t = g * W[m];
-    fp[m] = __fma_rn(w[m].u[0] + lam_u, c, -t);
-    fm[m] = __fma_rn(w[m].u[0] - lam_u, c, -t);
+    const double c = __fma_rn(-g, P[m], A.q(m, 0)), t = g * W[m];
+    fp[m] = __fma_rn(A.un(m) + lam_u, c, -t);
+    fm[m] = __fma_rn(A.un(m) - lam_u, c, -t);
   }
   const double r0 = 0.5 * wave(fp, fm, 4.0);
   // vorticity waves: t1 along +t2, t2 along -t1 (3D); 2D has the second alone
@@ -581,18 +650,18 @@ __device__ __forceinline__ void char_flux_f64(const Pt<double, ND> (&w)[6], cons
   if constexpr (ND == 3) {
 #pragma unroll
     for (int m = 0; m < 6; ++m) {
-      const double c = __fma_rn(-u[ND - 1], w[m].q[0], w[m].q[ND]);
-      fp[m] = (w[m].u[0] + lam_u) * c;
-      fm[m] = (w[m].u[0] - lam_u) * c;
+      const double c = __fma_rn(-u[ND - 1], A.q(m, 0), A.q(m, ND));
+      fp[m] = (A.un(m) + lam_u) * c;
+      fm[m] = (A.un(m) - lam_u) * c;
     }
     t1 = 0.5 * wave(fp, fm, 4.0 * rho2);
   }
   if constexpr (ND >= 2) {
 #pragma unroll
     for (int m = 0; m < 6; ++m) {
-      const double c = __fma_rn(u[1], w[m].q[0], -w[m].q[2]);
-      fp[m] = (w[m].u[0] + lam_u) * c;
-      fm[m] = (w[m].u[0] - lam_u) * c;
+      const double c = __fma_rn(u[1], A.q(m, 0), -A.q(m, 2));
+      fp[m] = (A.un(m) + lam_u) * c;
+      fm[m] = (A.un(m) - lam_u) * c;
     }
     t2 = 0.5 * wave(fp, fm, 4.0 * rho2);
   }
@@ -601,7 +670,7 @@ __device__ __forceinline__ void char_flux_f64(const Pt<double, ND> (&w)[6], cons
 #pragma unroll
   for (int m = 0; m < 6; ++m) {
     const double c = __fma_rn(gi, P[m], D[m]);
-    const double f = __fma_rn(w[m].u[0], c, __fma_rn(gi, W[m], w[m].p));
+    const double f = __fma_rn(A.un(m), c, __fma_rn(gi, W[m], A.p(m)));
     fp[m] = __fma_rn(lam_p, c, f);
     fm[m] = __fma_rn(-lam_p, c, f);
   }
@@ -609,7 +678,7 @@ __device__ __forceinline__ void char_flux_f64(const Pt<double, ND> (&w)[6], cons
 #pragma unroll
   for (int m = 0; m < 6; ++m) {
     const double c = __fma_rn(gi, P[m], -D[m]);
-    const double f = __fma_rn(w[m].u[0], c, __fma_rn(gi, W[m], -w[m].p));
+    const double f = __fma_rn(A.un(m), c, __fma_rn(gi, W[m], -A.p(m)));
     fp[m] = __fma_rn(lam_m, c, f);
     fm[m] = __fma_rn(-lam_m, c, f);
   }
@@ -825,16 +894,92 @@ __device__ __forceinline__ void char_flux_f32(const Pt<float, ND> (&w)[6], const
   fh[NV - 1] = e;
 }
 
+// Averaged state of a 1D interface (averaging.py:31-124) in the generated order.
+template <typename T, int AVG>
+struct Face1D {
+  T u, a, H, iden, ia;
+  __device__ __forceinline__ Face1D(const Pt<T, 1>& L, const Pt<T, 1>& R, const SP<T>& sp) {
+    if (AVG == AVG_ROE) {
+      T sL = sqrt(L.q[0]), sR = sqrt(R.q[0]);
+      T inv = L_(1.0) / (sL + sR);
+      u = (sL * L.u[0] + sR * R.u[0]) * inv;
+      T ke = L_(0.0) + u * u;
+      T h = ((L.q[2] + L.p) / sL + (R.q[2] + R.p) / sR) * inv;
+      a = sqrt(sp.g1 * (h - L_(0.5) * ke));
+    } else {
+      u = L_(0.5) * (L.u[0] + R.u[0]);
+      a = L_(0.5) * (L.a + R.a);
+    }
+    H = a * a / sp.g1 + L_(0.5) * u * u;
+    const T den = L_(2.0) * H - u * u;
+    iden = L_(1.0) / den;
+    ia = L_(1.0) / a;
+  }
+};
+
+// Reconstructed wave k of a 1D interface, 1D system of euler_eigensystem.py:85-99, H = a^2/(gama-1) +
+// u^2/2, waves (u-a, u, u+a), LLF speeds over points i, i+1 (shock_capturing.py:1000-1028).
+template <typename T, int SCH, int AVG>
+__device__ __forceinline__ T wave_1d(int k, const Pt<T, 1> (&w)[6], const SP<T>& sp, const Face1D<T, AVG>& fc) {
+  const Pt<T, 1>& L = w[2];
+  const Pt<T, 1>& R = w[3];
+  const T u0 = fc.u, a = fc.a, H = fc.H, iden = fc.iden, ia = fc.ia;
+  T l0, l1, l2, lam;
+  if (k == 0) {
+    l0 = u0 * (L_(2.0) * H + a * u0 - u0 * u0) * L_(0.5) * ia * iden;
+    l1 = (-H - a * u0 + L_(0.5) * u0 * u0) * ia * iden;
+    l2 = iden;
+    lam = sp.sfc * fmax(fabs(L.u[0] - L.a), fabs(R.u[0] - R.a));
+  } else if (k == 1) {
+    l0 = L_(2.0) * (H - u0 * u0) * iden;
+    l1 = L_(2.0) * u0 * iden;
+    l2 = -L_(2.0) * iden;
+    lam = sp.sfc * fmax(fabs(L.u[0]), fabs(R.u[0]));
+  } else {
+    l0 = u0 * (-L_(2.0) * H + a * u0 + u0 * u0) * L_(0.5) * ia * iden;
+    l1 = (H - a * u0 - L_(0.5) * u0 * u0) * ia * iden;
+    l2 = iden;
+    lam = sp.sfc * fmax(fabs(L.u[0] + L.a), fabs(R.u[0] + R.a));
+  }
+  T fp[6], fm[6];
+#pragma unroll
+  for (int m = 0; m < 6; ++m) {
+    const T F0 = w[m].q[1];
+    const T F1 = w[m].u[0] * w[m].q[1] + w[m].p;
+    const T F2 = w[m].u[0] * (w[m].q[2] + w[m].p);
+    T cs = l0 * w[m].q[0] + l1 * w[m].q[1] + l2 * w[m].q[2];
+    T cf = l0 * F0 + l1 * F1 + l2 * F2;
+    fp[m] = L_(0.5) * (cf + lam * cs);
+    fm[m] = L_(0.5) * (cf - lam * cs);
+  }
+  return recon_wave<T, SCH, true>(fp, fm, sp);
+}
+
+template <typename T>
+__device__ __forceinline__ void flux_1d(const T (&rec)[3], T u0, T a, T H, T (&fh)[3]) {
+  fh[0] = rec[0] + rec[1] + rec[2];
+  fh[1] = (u0 - a) * rec[0] + u0 * rec[1] + (u0 + a) * rec[2];
+  fh[2] = (H - u0 * a) * rec[0] + L_(0.5) * u0 * u0 * rec[1] + (H + u0 * a) * rec[2];
+}
+
 // Characteristic LLF flux at the interface between w[2] and w[3] of a 6-point window
 // (offsets -2..+3), local frame.  Restates shock_capturing.py:786-891 and 979-1028 with the
 // eigensystems of euler_eigensystem.py for k = e_0.
 template <typename T, int ND, int SCH, int AVG>
 __device__ __forceinline__ void char_flux(const Pt<T, ND> (&w)[6], const SP<T>& sp, T (&fh)[ND + 2]) {
-  if constexpr (sizeof(T) == 8) {
-    char_flux_f64<ND, SCH, AVG>(w, sp, fh);
+  if constexpr (sizeof(T) == 8 && !generated_order<ND, SCH>()) {
+    char_flux_f64<ND, SCH, AVG>(WindowF64<ND>{w}, sp, fh);
     return;
-  } else if constexpr (ND >= 2 && SCH != SCH_TENO6) {
+  } else if constexpr (sizeof(T) == 4 && ND >= 2 && SCH != SCH_TENO6) {
     char_flux_f32<ND, SCH, AVG>(w, sp, fh);
+    return;
+  }
+  if constexpr (ND == 1) {
+    const Face1D<T, AVG> fc(w[2], w[3], sp);
+    T rec[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) rec[k] = wave_1d<T, SCH, AVG>(k, w, sp, fc);
+    flux_1d(rec, fc.u, fc.a, fc.H, fh);
     return;
   }
   constexpr int NV = ND + 2;
@@ -868,44 +1013,6 @@ __device__ __forceinline__ void char_flux(const Pt<T, ND> (&w)[6], const SP<T>& 
   T lam_m = sfc * fmax(fabs(L.u[0] - L.a), fabs(R.u[0] - R.a));
 
   T rec[NV];
-  if (ND == 1) {
-    // 1D system, euler_eigensystem.py:85-99, H = a^2/(gama-1) + u^2/2, waves (u-a, u, u+a)
-    const T u0 = u[0];
-    const T H = a * a / g1 + L_(0.5) * u0 * u0;
-    const T den = L_(2.0) * H - u0 * u0;
-    const T iden = L_(1.0) / den, ia = L_(1.0) / a;
-    T Lm[3][3];
-    Lm[0][0] = u0 * (L_(2.0) * H + a * u0 - u0 * u0) * L_(0.5) * ia * iden;
-    Lm[0][1] = (-H - a * u0 + L_(0.5) * u0 * u0) * ia * iden;
-    Lm[0][2] = iden;
-    Lm[1][0] = L_(2.0) * (H - u0 * u0) * iden;
-    Lm[1][1] = L_(2.0) * u0 * iden;
-    Lm[1][2] = -L_(2.0) * iden;
-    Lm[2][0] = u0 * (-L_(2.0) * H + a * u0 + u0 * u0) * L_(0.5) * ia * iden;
-    Lm[2][1] = (H - a * u0 - L_(0.5) * u0 * u0) * ia * iden;
-    Lm[2][2] = iden;
-    const T lam[3] = {lam_m, lam_u, lam_p};
-    T fp[3][6], fmn[3][6];
-#pragma unroll
-    for (int m = 0; m < 6; ++m) {
-      const T F0 = w[m].q[1];
-      const T F1 = w[m].u[0] * w[m].q[1] + w[m].p;
-      const T F2 = w[m].u[0] * (w[m].q[2] + w[m].p);
-#pragma unroll
-      for (int k = 0; k < 3; ++k) {
-        T cs = Lm[k][0] * w[m].q[0] + Lm[k][1] * w[m].q[1] + Lm[k][2] * w[m].q[2];
-        T cf = Lm[k][0] * F0 + Lm[k][1] * F1 + Lm[k][2] * F2;
-        fp[k][m] = L_(0.5) * (cf + lam[k] * cs);
-        fmn[k][m] = L_(0.5) * (cf - lam[k] * cs);
-      }
-    }
-#pragma unroll
-    for (int k = 0; k < 3; ++k) rec[k] = recon_wave<T, SCH>(fp[k], fmn[k], sp);
-    fh[0] = rec[0] + rec[1] + rec[2];
-    fh[1] = (u0 - a) * rec[0] + u0 * rec[1] + (u0 + a) * rec[2];
-    fh[2] = (H - u0 * a) * rec[0] + L_(0.5) * u0 * u0 * rec[1] + (H + u0 * a) * rec[2];
-    return;
-  }
   // ---- 2D / 3D with k = e_0: waves 0..ND-1 move with u_n, ND with u_n + a, ND+1 with u_n - a
   const T ia = L_(1.0) / a, ia2 = ia * ia, irho = L_(1.0) / rho;
   T ke = L_(0.0);
@@ -968,7 +1075,7 @@ __device__ __forceinline__ void char_flux(const Pt<T, ND> (&w)[6], const SP<T>& 
     }
   }
 #pragma unroll
-  for (int k = 0; k < NV; ++k) rec[k] = recon_wave<T, SCH>(fp[k], fmn[k], sp);
+  for (int k = 0; k < NV; ++k) rec[k] = recon_wave<T, SCH, true>(fp[k], fmn[k], sp);
   // back to physical space with the REV columns (k = e_0)
   const T rp = rec[ND] + rec[ND + 1], rm = rec[ND] - rec[ND + 1];
   const T F0 = rec[0] + alf * rp;
@@ -1056,8 +1163,13 @@ __device__ __forceinline__ void hllc_flux(const Pt<T, ND> (&w)[6], const SP<T>& 
   T rl[NV], rr[NV];
 #pragma unroll
   for (int k = 0; k < NV; ++k) {
-    rl[k] = recon5<T, SCH>(cs[k][0], cs[k][1], cs[k][2], cs[k][3], cs[k][4], sp);
-    rr[k] = recon5<T, SCH>(cs[k][5], cs[k][4], cs[k][3], cs[k][2], cs[k][1], sp);
+    if constexpr (sizeof(T) == 8 && generated_order<ND, SCH>()) {
+      rl[k] = recon5_ieee<SCH>(cs[k][0], cs[k][1], cs[k][2], cs[k][3], cs[k][4], sp.teno_eps, sp.teno_ct);
+      rr[k] = recon5_ieee<SCH>(cs[k][5], cs[k][4], cs[k][3], cs[k][2], cs[k][1], sp.teno_eps, sp.teno_ct);
+    } else {
+      rl[k] = recon5<T, SCH>(cs[k][0], cs[k][1], cs[k][2], cs[k][3], cs[k][4], sp);
+      rr[k] = recon5<T, SCH>(cs[k][5], cs[k][4], cs[k][3], cs[k][2], cs[k][1], sp);
+    }
   }
   // REV columns (k = e_0): characteristic -> conserved, both sides
   T qL[NV], qR[NV];
@@ -1324,7 +1436,7 @@ __device__ __forceinline__ void char_flux_curv(const PtC<T, ND> (&w)[6], const S
     }
   } else {
 #pragma unroll
-    for (int c = 0; c < NV; ++c) rec[c] = recon_wave<T, SCH>(fp[c], fmn[c], sp);
+    for (int c = 0; c < NV; ++c) rec[c] = recon_wave<T, SCH, generated_order<ND, SCH>()>(fp[c], fmn[c], sp);
   }
   // REV: 2D columns (1, u, phi/g1), rho (0, t, t.u) with t = (k1, -k0), and the acoustic
   // pair alf (1, u +- a k, h0 +- a th); 3D vorticity columns give u (k.r) + rho (k x r) and

@@ -52,7 +52,7 @@ struct RLayout {
   double *q, *o;       // [3][most]: state and register
   double* halo;        // [2 parities][2 sides][RH points][3]: the neighbours' outer points
   T *F;                // [3][most + 1]: flux at the left face of point i (FP64: its three reconstructed waves)
-  T *V;                // FP64: [3][most + 1]: averaged u, a, 1 / a of the face
+  T *V;                // FP64: [3][most + 1]: averaged u, a, 1 / a (or H) of the face
   T* P;                // [8][most + 2 RH]: rho, m, E, u, p, a (, sqrt(rho), H in FP64) from point -RH
   __device__ RLayout(unsigned char* sm, int most) {
     q = reinterpret_cast<double*>(sm);
@@ -115,10 +115,11 @@ __device__ __forceinline__ void get_prims(const T* P, int stride, Pt<T, 1>& w) {
 
 // FP64: the interfaces of a CTA are few (a warp of them), and an FP64 instruction's result takes
 // several times the 16 cycles of its issue, so one warp leaves the pipe mostly waiting.  Each
-// wave of an interface goes to its own warp (char_flux_f64's rows for one dimension): k = 0 entropy,
-// 1 u + a, 2 u - a.  The point's own thread turns the waves of its two faces into fluxes.
+// wave of an interface goes to its own warp, and the point's own thread turns the waves of its two
+// faces into fluxes.  WENO takes char_flux_f64's rows for one dimension, k = 0 entropy, 1 u + a, 2 u - a
+// (the 400-point shock tube's 50 steps: 0.46 ms, and 0.65 ms with wave_1d's divisions), TENO wave_1d.
 template <int SCH>
-__device__ __forceinline__ double wave_1d(int k, const Pt<double, 1> (&w)[6], const SP<double>& sp, double u, double a,
+__device__ __forceinline__ double wave_1d_f64(int k, const Pt<double, 1> (&w)[6], const SP<double>& sp, double u, double a,
                                           double ia, double ke) {
   const Pt<double, 1>& L = w[2];
   const Pt<double, 1>& R = w[3];
@@ -137,20 +138,9 @@ __device__ __forceinline__ double wave_1d(int k, const Pt<double, 1> (&w)[6], co
     fm[m] = __fma_rn(w[m].u[0] - lam, c, t);
   }
   const double s2 = k == 0 ? 4.0 : 16.0 * a * a;
-  if constexpr (SCH == SCH_TENO6) {
-    const double sc = k == 0 ? 2.0 : 4.0 * a, isc = k == 0 ? 0.5 : 0.25 * ia;
-#pragma unroll
-    for (int m = 0; m < 6; ++m) {
-      fp[m] *= isc;
-      fm[m] *= isc;
-    }
-    return sc * (recon6<double, 1>(fp[0], fp[1], fp[2], fp[3], fp[4], fp[5], sp) +
-                 recon6<double, -1>(fm[0], fm[1], fm[2], fm[3], fm[4], fm[5], sp));
-  } else {
-    const ReconEps e = recon_eps<SCH>(sp.teno_eps, s2);
-    return recon5_f64<SCH>(fp[0], fp[1], fp[2], fp[3], fp[4], e, sp.teno_ct, sp.teno_ct_f) +
-           recon5_f64<SCH>(fm[5], fm[4], fm[3], fm[2], fm[1], e, sp.teno_ct, sp.teno_ct_f);
-  }
+  const ReconEps e = recon_eps<SCH>(sp.teno_eps, s2);
+  return recon5_f64<SCH>(fp[0], fp[1], fp[2], fp[3], fp[4], e, sp.teno_ct, sp.teno_ct_f) +
+         recon5_f64<SCH>(fm[5], fm[4], fm[3], fm[2], fm[1], e, sp.teno_ct, sp.teno_ct_f);
 }
 
 // T = double: the FP64 path.  T = float: the FP32-residual path -- the state and RK register
@@ -246,13 +236,21 @@ __global__ void __launch_bounds__(RT) k_resident_1d(const Resident1D* __restrict
           get_prims<T, AVG>(P, PS, w[m]);
         }
         if constexpr (!F32) {
-          double u[1], a, ia, rho2, ke;
-          face_average_f64<1, AVG>(w[2], w[3], sp.g1, u, a, ia, rho2, ke);
-          L.F[wave * (most + 1) + i] = wave_1d<SCH>(wave, w, sp, u[0], a, ia, ke);
+          double u, a, x;  // x: 1 / a, or H in the generated order
+          if constexpr (generated_order<1, SCH>()) {
+            const Face1D<T, AVG> fc(w[2], w[3], sp);
+            L.F[wave * (most + 1) + i] = wave_1d<T, SCH, AVG>(wave, w, sp, fc);
+            u = fc.u, a = fc.a, x = fc.H;
+          } else {
+            double uu[1], rho2, ke;
+            face_average_f64<1, AVG>(w[2], w[3], sp.g1, uu, a, x, rho2, ke);
+            u = uu[0];
+            L.F[wave * (most + 1) + i] = wave_1d_f64<SCH>(wave, w, sp, u, a, x, ke);
+          }
           if (wave == 0) {
-            L.V[i] = u[0];
+            L.V[i] = u;
             L.V[most + 1 + i] = a;
-            L.V[2 * (most + 1) + i] = ia;
+            L.V[2 * (most + 1) + i] = x;
           }
           continue;
         }
@@ -274,12 +272,15 @@ __global__ void __launch_bounds__(RT) k_resident_1d(const Resident1D* __restrict
             for (int v = 0; v < 3; ++v) face[e][v] = F[v * (most + 1)];
           } else {
             const double* V = L.V + i + e;
-            const double u = V[0], a = V[most + 1], ia = V[2 * (most + 1)];
-            const double r0 = 0.5 * F[0], rp = F[most + 1], rm = F[2 * (most + 1)];
-            const double S = 0.25 * (rp + rm), Bm = 0.25 * (rp - rm), F0 = __fma_rn(ia, S, r0);
-            face[e][0] = F0;
-            face[e][1] = __fma_rn(u, F0, Bm);
-            face[e][2] = __fma_rn(0.5 * (u * u), F0, __fma_rn(a * sp.ig1, S, u * Bm));
+            const double rec[3] = {F[0], F[most + 1], F[2 * (most + 1)]}, u = V[0], a = V[most + 1], x = V[2 * (most + 1)];
+            if constexpr (generated_order<1, SCH>()) {
+              flux_1d(rec, u, a, x, face[e]);
+            } else {
+              const double S = 0.25 * (rec[1] + rec[2]), Bm = 0.25 * (rec[1] - rec[2]), F0 = __fma_rn(x, S, 0.5 * rec[0]);
+              face[e][0] = F0;
+              face[e][1] = __fma_rn(u, F0, Bm);
+              face[e][2] = __fma_rn(0.5 * (u * u), F0, __fma_rn(a * sp.ig1, S, u * Bm));
+            }
           }
         }
 #pragma unroll

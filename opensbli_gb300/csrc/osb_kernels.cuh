@@ -437,7 +437,7 @@ __global__ void __launch_bounds__(SWEEP_THREADS, sizeof(T) == 4 ? 3 : 1)
     int id = base + (j0 - 4 + m) * s;
 #pragma unroll
     for (int f = 0; f < NF; ++f) set_field(w[m], f, ld_field<T, ND, D, CURV>(b, f, id));
-    make_pt<T, ND>(w[m], gm);
+    make_pt<T, ND, generated_order<ND, SCH>()>(w[m], gm);
   }
   T fprev[NV];
 #pragma unroll
@@ -454,7 +454,7 @@ __global__ void __launch_bounds__(SWEEP_THREADS, sizeof(T) == 4 ? 3 : 1)
     for (int m = 0; m < 5; ++m) w[m] = w[m + 1];
 #pragma unroll
     for (int f = 0; f < NF; ++f) set_field(w[5], f, ring[cur][f][tid]);
-    make_pt<T, ND>(w[5], gm);
+    make_pt<T, ND, generated_order<ND, SCH>()>(w[5], gm);
     const int id = base + j * s;
     T oh[NV], ol[NV];
     if (rd && j >= j0) {
@@ -621,7 +621,7 @@ __global__ void __launch_bounds__(32 * XWARPS, sizeof(T) == 4 ? (CURV ? 4 : 6) :
     }
 #pragma unroll
     for (int f = 0; f < NF; ++f) set_field(w[m], f, t.in[f][lane][(m - 1) % XCOLS]);
-    make_pt<T, ND>(w[m], gm);
+    make_pt<T, ND, generated_order<ND, SCH>()>(w[m], gm);
   }
   for (int j = s0 - 1; j < s1; ++j) {
     const int rc = j - s0 + 6;  // input column of the new point j + 3
@@ -637,7 +637,7 @@ __global__ void __launch_bounds__(32 * XWARPS, sizeof(T) == 4 ? (CURV ? 4 : 6) :
     for (int m = 0; m < 5; ++m) w[m] = w[m + 1];
 #pragma unroll
     for (int f = 0; f < NF; ++f) set_field(w[5], f, t.in[f][lane][rc % XCOLS]);
-    make_pt<T, ND>(w[5], gm);
+    make_pt<T, ND, generated_order<ND, SCH>()>(w[5], gm);
     T fh[NV];
     if constexpr (CURV) {
       char_flux_curv<T, ND, SCH, AVG>(w, sp, fh);

@@ -178,6 +178,8 @@ static __device__ const double teno5_rows[8][4] = {
     OSB_TENO5_ROW(11.0, 8.0, 1.0, 20.0)};
 #undef OSB_TENO5_ROW
 
+// Blocks whose flux keeps the generated order of operations (projections, primitives, divisions and
+// indicators; recon5_ieee says why), in both precisions.
 template <int ND, int SCH>
 __host__ __device__ constexpr bool generated_order() {
   return ND <= 2 && (SCH == SCH_TENO5 || SCH == SCH_TENO6);
@@ -185,7 +187,7 @@ __host__ __device__ constexpr bool generated_order() {
 
 // Fifth-order reconstruction in the generated order with IEEE divisions, FP64.  It serves
 //   - values beyond the range of recon5_f64's common denominator,
-//   - TENO5 on 1D and 2D blocks (generated_order; TENO6 keeps it too).  A front in exactly uniform gas is symmetric
+//   - TENO5 on 1D and 2D blocks (generated_order; TENO6 keeps the order too).  A front in exactly uniform gas is symmetric
 //     at first, so the outer indicators of a five-point window tie while the middle one is zero to
 //     rounding: tau is then the rounding of b0 - b2, and whether it is exactly zero decides if TENO5
 //     keeps the outer stencils.  Another order of the same operations moves a shock tube by 1e-7
@@ -474,7 +476,8 @@ struct Pt {
   T p, a;
 };
 
-template <typename T, int ND>
+// GEN: the sweep keeps the generated order (generated_order).
+template <typename T, int ND, bool GEN = false>
 __device__ __forceinline__ void make_pt(Pt<T, ND>& s, T gm) {
   T rho = s.q[0];
   T ir = L_(1.0) / rho;
@@ -491,8 +494,20 @@ __device__ __forceinline__ void make_pt(Pt<T, ND>& s, T gm) {
 // FP32 2D: the kinetic energy as a sum of two rounded squares, which does not depend on the order of
 // the components: the persistent stage forms a point's primitives once for both directions, the
 // sweeps in each direction's own frame, and they agree bit for bit.
-template <typename T, int ND>
+template <typename T, int ND, bool GEN = false>
 __device__ __forceinline__ void make_pt(Pt<float, 2>& s, float gm) {
+  if constexpr (GEN) {
+    const float rho = s.q[0], ir = 1.0f / rho;
+    float ke = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      s.u[i] = s.q[1 + i] * ir;
+      ke += s.u[i] * s.u[i];
+    }
+    s.p = (gm - 1.0f) * (s.q[3] - 0.5f * rho * ke);
+    s.a = sqrtf(gm * s.p * ir);
+    return;
+  }
   const float ir = 1.0f / s.q[0];
   s.u[0] = __fmul_rn(s.q[1], ir);
   s.u[1] = __fmul_rn(s.q[2], ir);
@@ -508,7 +523,7 @@ struct Pt<double, ND> {
   double q[ND + 2], u[ND];
   double p, a, s, H;  // s = sqrt(rho), H = (E + p) / rho
 };
-template <typename T, int ND>
+template <typename T, int ND, bool GEN = false>
 __device__ __forceinline__ void make_pt(Pt<double, ND>& s, double gm) {
   if constexpr (ND <= 2) {  // the generated order (recon5_ieee)
     const double rho = s.q[0], ir = 1.0 / rho;
@@ -970,7 +985,7 @@ __device__ __forceinline__ void char_flux(const Pt<T, ND> (&w)[6], const SP<T>& 
   if constexpr (sizeof(T) == 8 && !generated_order<ND, SCH>()) {
     char_flux_f64<ND, SCH, AVG>(WindowF64<ND>{w}, sp, fh);
     return;
-  } else if constexpr (sizeof(T) == 4 && ND >= 2 && SCH != SCH_TENO6) {
+  } else if constexpr (sizeof(T) == 4 && ND >= 2 && SCH != SCH_TENO6 && !generated_order<ND, SCH>()) {
     char_flux_f32<ND, SCH, AVG>(w, sp, fh);
     return;
   }
@@ -1268,7 +1283,7 @@ struct PtC {
   T J;          // det(d x / d xi)
 };
 
-template <typename T, int ND>
+template <typename T, int ND, bool GEN = false>
 __device__ __forceinline__ void make_pt(PtC<T, ND>& s, T gm) {
   T rho = s.q[0];
   T ir = L_(1.0) / rho;

@@ -3,6 +3,7 @@
 // instantiations build in parallel.
 #include <algorithm>
 
+#include "osb_flux64.cuh"
 #include "osb_internal.h"
 
 #ifndef OSB_T
@@ -46,10 +47,29 @@ int launch_sweep(osb_ctx* c, const BlockK& k, const SchemeParams& sp, int N, int
   return launch_sweep_k<T, ND, D, SCH, AVG, CURV, false, FLX>(c, k, sp, N, other, RkFuse{});
 }
 
+// FP64 LLF sweep of a 2D / 3D Cartesian block along D (k_flux_tile).
+template <int ND, int D, int SCH, int AVG>
+int launch_tile(osb_ctx* c, Block& bl, const SchemeParams& sp) {
+  using Tl = F64Tile<D>;
+  const BlockK& k = bl.k;
+  auto kern = k_flux_tile<ND, D, SCH, AVG>;
+  constexpr size_t smem = F64Fields<ND, D, AVG>::bytes;
+  OSB_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const long lines = (long)k.n[0] * k.n[1] * k.n[2] / k.n[D];
+  const int parts = (k.n[D] + Tl::NI - 2) / (Tl::NI - 1), pts = (k.n[D] + parts - 1) / parts;
+  const long gx = (lines + Tl::NC - 1) / Tl::NC;
+  if (parts > 65535 || (D > 0 && lines / k.n[0] > 65535)) return fail(OSB_ENOTSUP, "block too large for the sweep grid");
+  timing_begin(c, D == 0 ? FAM_FLUX_X : D == 1 ? FAM_FLUX_Y : FAM_FLUX_Z);
+  kern<<<dim3((unsigned)gx, (unsigned)parts), F64T, smem, c->stream>>>(k, sp, pts, D == 0 ? 1 : 0);
+  timing_end(c);
+  c->launches++;
+  return OSB_OK;
+}
+
 // x sweep (writes R), then y[, z] sweeps (accumulate); with rf (FP32 path, 2D/3D) the last
 // sweep applies the RK update instead of storing the residual.
 template <typename T, int ND, int SCH, int AVG, bool CURV, int FLX = 0>
-int launch_flux(osb_ctx* c, Block& bl, const SchemeParams& sp, const RkFuse* rf) {
+int launch_lines(osb_ctx* c, Block& bl, const SchemeParams& sp, const RkFuse* rf) {
   BlockK& k = bl.k;
   cudaStream_t st = c->stream;
   // x sweep (writes R)
@@ -95,6 +115,28 @@ int launch_flux(osb_ctx* c, Block& bl, const SchemeParams& sp, const RkFuse* rf)
     c->launches++;
   }
   return OSB_OK;
+}
+
+// FP64 LLF blocks by tiles or by lines, all others by lines.
+template <typename T, int ND, int SCH, int AVG, bool CURV, int FLX = 0>
+int launch_flux(osb_ctx* c, Block& bl, const SchemeParams& sp, const RkFuse* rf) {
+  // FP64: a thread per interface beats a thread per line segment on blocks that leave SMs idle or in
+  // one unfinished wave, and holds 16 warps per SM against 8: WENO5-Z 2D 97 x 120 (4 steps) 2.1 and 9.1 ms,
+  // 2000 x 2000 116 and 116 ms; 3D 16^3 3.7 and 11.8, 64^3 19.0 and 20.1, 128^3 (1 step) 31.5 and 32.8 ms; TENO6
+  // 128^3 72.6 and 76.9 ms.  TENO5, with the least arithmetic per staged value (3D; 2D: divisions that 8
+  // warps hide as well), turns: 3D 48^3 4.8 and 8.2 ms, 64^3 11.4 and 12.1, but 96^3 8.1 and 7.7; 2D
+  // 97 x 120 4.8 and 21.1, 1000 x 1000 71.9 and 76.7, but 2000 x 2000 277 and 273.
+  constexpr bool TILE = sizeof(T) == 8 && ND >= 2 && !CURV && FLX == 0, ALWAYS = TILE && SCH != SCH_TENO5;
+  if constexpr (TILE) {
+    if (ALWAYS || (long)bl.k.n[0] * bl.k.n[1] * bl.k.n[2] < (ND == 3 ? 512000L : 2000000L)) {
+      int rc = launch_tile<ND, 0, SCH, AVG>(c, bl, sp);
+      if (rc == OSB_OK) rc = launch_tile<ND, 1, SCH, AVG>(c, bl, sp);
+      if constexpr (ND == 3)
+        if (rc == OSB_OK) rc = launch_tile<ND, 2, SCH, AVG>(c, bl, sp);
+      return rc;
+    }
+  }
+  if constexpr (!ALWAYS) return launch_lines<T, ND, SCH, AVG, CURV, FLX>(c, bl, sp, rf);
 }
 
 // HLLC-LM flux (Cartesian 2D / 3D blocks, fifth-order reconstructions): the sweeps do not carry

@@ -68,3 +68,23 @@ def test_sweeps_fp32_lines(built_lib, oracle_lib, sizes, scheme):
         # TENO5's cut-off may flip where it is within FP32 rounding of its threshold: a few points
         bad = int(np.count_nonzero(d > 2e-4 * scale))
         assert bad <= (d.size // 500 if scheme == abi.SCHEME_TENO5 else 0), (v, bad, float(d.max()) / scale)
+
+
+# k_flux_tile: 63 points of 8 rows along x, 15 points of 32 lines along y and z
+@pytest.mark.parametrize("sizes", [(63, 8), (64, 9), (127, 33), (31, 16), (6, 7), (63, 8, 6), (33, 15, 16), (65, 7, 31)])
+@pytest.mark.parametrize("scheme", [abi.SCHEME_WENO5_JS, abi.SCHEME_WENO5_Z, abi.SCHEME_TENO5, abi.SCHEME_TENO6])
+@pytest.mark.parametrize("avg", [abi.AVG_ROE, abi.AVG_SIMPLE])
+def test_sweeps_fp64_tiles(built_lib, oracle_lib, sizes, scheme, avg):
+    if len(sizes) == 3:
+        spec, q = _block(sizes, scheme, abi.VISC_NONE, 13, minf=1.25)
+    else:
+        spec, q = problems.kh(sizes=sizes, scheme=scheme)
+        rng = np.random.default_rng(13)
+        q = [a * (1.0 + 1e-2 * rng.standard_normal(a.shape)) for a in q]
+    spec.averaging = avg
+    got, ref, _, _ = _residuals(spec, q, "fp64")
+    sl = spec.interior()
+    mom = range(1, 1 + len(sizes))
+    for v in range(spec.nvars):
+        scale = max(float(np.max(np.abs(ref[w][sl]))) for w in (mom if v in mom else (v,)))
+        assert float(np.max(np.abs(got[v][sl] - ref[v][sl]))) < 1e-12 * scale, v

@@ -318,7 +318,8 @@ __global__ void __launch_bounds__(RT) k_resident_1d(const Resident1D* __restrict
           if (i >= n - RH && linked[1]) ph[1][hal(parity ^ 1, 0, n - 1 - i, v)] = qv;
         }
       }
-      cl.sync();  // also this CTA's barrier; after the last one nobody writes to a neighbour any more
+      if (cs == 1) __syncthreads();
+      else cl.sync();  // also this CTA's barrier; after the last one nobody writes to a neighbour any more
       parity ^= 1;
     }
   }
@@ -349,7 +350,9 @@ __global__ void __launch_bounds__(RT) k_resident_1d(const Resident1D* __restrict
 
 // Points are split over the smallest power of two of CTAs that leaves each a warp of interfaces
 // (31 points), up to the largest cluster the GPU grants: below a warp an FP64 instruction costs the
-// same.  400 points: 16 CTAs of 25.  Contexts of many blocks take smaller clusters (no fewer than
+// same.  400 points: 16 CTAs of 25.  FP32: 125 points, four warps, which take as long as one (50
+// points, 20 steps: one CTA 0.160 ms, two 0.177; 400: 4 CTAs 0.17, 2 0.20, 1 0.30).  One CTA alone is no
+// cluster: a plain launch and CTA barriers.  Contexts of many blocks take smaller clusters (no fewer than
 // two CTAs where a block has more than 31 points: one holds about 1 600), enough to fill the SMs.
 template <typename T, int SCH, int AVG>
 int launch_resident(osb_ctx* c, const Resident1D* dev, int nblocks, int maxN, double dt, int nsteps) {
@@ -364,21 +367,21 @@ int launch_resident(osb_ctx* c, const Resident1D* dev, int nblocks, int maxN, do
   }
   auto points = [&](int C) { return (maxN + C - 1) / C; };
   int C = 1;
-  while (C < RC && points(C) > 31) C *= 2;
+  while (C < RC && points(C) > (sizeof(T) == 8 ? 31 : 125)) C *= 2;
   while (C > 2 && (long)nblocks * (C / 2) >= 2L * c->sm_count) C /= 2;
   auto kern = k_resident_1d<T, SCH, AVG>;
-  OSB_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  if (C > 8) OSB_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
   cudaLaunchConfig_t cfg{};
   cudaLaunchAttribute at{};
   at.id = cudaLaunchAttributeClusterDimension;
   cfg.attrs = &at;
-  cfg.numAttrs = 1;
   cfg.stream = c->stream;
   int most = 0;
   for (;; C /= 2) {
     most = std::max(points(C), 4 * RH);  // a smaller block's share: below 2 (2 RH) points each
     const size_t smem = RLayout<T>::bytes(most);
-    OSB_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (smem > 48 * 1024) OSB_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    cfg.numAttrs = C > 1 ? 1 : 0;
     at.val.clusterDim.x = (unsigned)C;
     at.val.clusterDim.y = at.val.clusterDim.z = 1;
     cfg.gridDim = dim3((unsigned)(nblocks * C));

@@ -248,26 +248,57 @@ __device__ __forceinline__ void filter_flux(const Pt<T, 3> (&w)[4], const SP<T>&
   fh[4] = phi / g1 * rec[0] + rho * u[2] * rec[1] - rho * u[1] * rec[2] + alf * h0 * rp + alf * u[0] * a * rmn;
 }
 
+// Whether a filter flux acts at interface i+1/2 (id: point i, s: step along the direction): its stencil
+// i-3..i+2 sees a kappa above Ducros_check.
+template <typename T>
+__device__ __forceinline__ bool filter_on(const T* __restrict__ kappa, int id, int s, T check) {
+  T km = kappa[id - 3 * s];
+#pragma unroll
+  for (int m = -2; m <= 2; ++m) km = fmax(km, kappa[id + m * s]);
+  return km > check;
+}
+
 // Filter fluxes along D at interfaces i+1/2, i = -1..N-1, transverse interior; F[v] at the
-// index of point i.  Interfaces whose stencil i-3..i+2 sees no kappa above Ducros_check get 0.
+// index of point i, only where filter_on holds (k_filter_apply asks it again).
+//
+// Few interfaces are on (8 % of a supersonic vortex at Ducros_check 0.05), but they are spread over a
+// quarter of the warps, and the flux takes 900 instructions: a CTA lists the ones that are on among
+// FQ per thread and works the list off in whole warps (128^3, 2 steps: 1.45 -> 1.35 ms).  Zeros are not
+// written for the others (60 bytes per point).  FQ 2, 4, 8, 16: 128^3 1.35, 1.34, 1.35, 1.36 ms, 64^3 FP32
+// 0.53, 0.54, 0.57, 0.64, 33^3 FP64 1.6, 1.9, 2.4, 3.3: small blocks want the CTAs.
+constexpr int FQ = 2;
 template <typename T, int D>
-__global__ void k_filter_flux(BlockK b, SchemeParams spd, const T* __restrict__ kappa, T check, T* F0, T* F1, T* F2,
-                              T* F3, T* F4) {
+__global__ void __launch_bounds__(FT) k_filter_flux(BlockK b, SchemeParams spd, const T* __restrict__ kappa, T check,
+                                                    T* F0, T* F1, T* F2, T* F3, T* F4) {
   const SP<T> sp(spd);
+  __shared__ int list[FQ * FT], count;
   int e[3] = {b.n[0], b.n[1], b.n[2]};
   e[D] += 1;
-  const int total = e[0] * e[1] * e[2];
+  const int total = e[0] * e[1] * e[2], lane = threadIdx.x & 31;
   const int s = b.st[D];
   T* F[5] = {F0, F1, F2, F3, F4};
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
-    int c[3] = {t % e[0], (t / e[0]) % e[1], t / (e[0] * e[1])};
-    c[D] -= 1;
-    const int id = lin(b, c[0], c[1], c[2]);
-    T km = kappa[id - 3 * s];
-#pragma unroll
-    for (int m = -2; m <= 2; ++m) km = fmax(km, kappa[id + m * s]);
-    T fh[5] = {L_(0.0), L_(0.0), L_(0.0), L_(0.0), L_(0.0)};
-    if (km > check) {
+  for (long t0 = (long)blockIdx.x * (FQ * FT); t0 < total; t0 += (long)gridDim.x * (FQ * FT)) {
+    if (threadIdx.x == 0) count = 0;
+    __syncthreads();
+    for (int j = 0; j < FQ; ++j) {
+      const long t = t0 + j * FT + threadIdx.x;
+      int id = 0;
+      bool on = false;
+      if (t < total) {
+        int c[3] = {(int)t % e[0], ((int)t / e[0]) % e[1], (int)t / (e[0] * e[1])};
+        c[D] -= 1;
+        id = lin(b, c[0], c[1], c[2]);
+        on = filter_on<T>(kappa, id, s, check);
+      }
+      const unsigned m = __ballot_sync(0xffffffffu, on);
+      int base = 0;
+      if (lane == 0 && m) base = atomicAdd(&count, __popc(m));
+      base = __shfl_sync(0xffffffffu, base, 0);
+      if (on) list[base + __popc(m & ((1u << lane) - 1u))] = id;
+    }
+    __syncthreads();
+    for (int k = threadIdx.x; k < count; k += FT) {
+      const int id = list[k];
       Pt<T, 3> w[4];
 #pragma unroll
       for (int m = 0; m < 4; ++m) {
@@ -276,10 +307,12 @@ __global__ void k_filter_flux(BlockK b, SchemeParams spd, const T* __restrict__ 
         for (int lv = 0; lv < 5; ++lv) w[m].q[lv] = ld_q<T>(b, gvar_fwd<3, D>(lv), pid);
         make_pt<T, 3>(w[m], sp.gama);
       }
+      T fh[5];
       filter_flux<T>(w, sp, fh);
-    }
 #pragma unroll
-    for (int lv = 0; lv < 5; ++lv) F[gvar_fwd<3, D>(lv)][id] = fh[lv];
+      for (int lv = 0; lv < 5; ++lv) F[gvar_fwd<3, D>(lv)][id] = fh[lv];
+    }
+    __syncthreads();  // the next round starts the list anew
   }
 }
 
@@ -530,7 +563,7 @@ struct FilterFluxes {
 };
 
 template <typename T>
-__global__ void k_filter_apply(BlockK b, const T* __restrict__ kappa, FilterFluxes<T> F, double dt, T select) {
+__global__ void k_filter_apply(BlockK b, const T* __restrict__ kappa, FilterFluxes<T> F, double dt, T select, T check) {
   const int n0 = b.n[0], n1 = b.n[1], n2 = b.n[2];
   const int total = n0 * n1 * n2;
   const int sx = b.st[0], sy = b.st[1], sz = b.st[2];
@@ -551,12 +584,23 @@ __global__ void k_filter_apply(BlockK b, const T* __restrict__ kappa, FilterFlux
       km = fmax(km, kappa[c - sz]);
       if (!(km >= select)) continue;  // mask 0: the state is unchanged
     }
+    // the fluxes of the point's six faces that are not zero (k_filter_flux; the TVD filter writes all)
+    bool on[3][2];
+    const int st[3] = {sx, sy, sz};
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      on[d][0] = !kappa || filter_on<T>(kappa, c - st[d], st[d], check);
+      on[d][1] = !kappa || filter_on<T>(kappa, c, st[d], check);
+    }
 #pragma unroll
     for (int v = 0; v < 5; ++v) {
       const T* f0 = F.f[v];
       const T* f1 = F.f[5 + v];
       const T* f2 = F.f[10 + v];
-      const T inc = -(-f0[c - sx] + f0[c]) * i0 - (-f2[c - sz] + f2[c]) * i2 - (-f1[c - sy] + f1[c]) * i1;
+      const T x0 = on[0][0] ? f0[c - sx] : L_(0.0), x1 = on[0][1] ? f0[c] : L_(0.0);
+      const T y0 = on[1][0] ? f1[c - sy] : L_(0.0), y1 = on[1][1] ? f1[c] : L_(0.0);
+      const T z0 = on[2][0] ? f2[c - sz] : L_(0.0), z1 = on[2][1] ? f2[c] : L_(0.0);
+      const T inc = -(-x0 + x1) * i0 - (-z0 + z1) * i2 - (-y0 + y1) * i1;
       if constexpr (sizeof(T) == 8) {
         b.q[v][c] = inc * dt * 1.0 + b.q[v][c];
       } else {
@@ -603,7 +647,7 @@ int tvd_filter_t(osb_ctx* c, Block& bl, double dt) {
   k_tvd_flux<T, 2><<<g2, TVD_TH, 0, c->stream>>>(k, gm, kap, snap, fmax, F[10], F[11], F[12], F[13], F[14]);
   FilterFluxes<T> Fd;
   for (int a = 0; a < 15; ++a) Fd.f[a] = F[a];
-  k_filter_apply<T><<<grid_for(c, n, FT), FT, 0, c->stream>>>(k, nullptr, Fd, dt, (T)0);
+  k_filter_apply<T><<<grid_for(c, n, FT), FT, 0, c->stream>>>(k, nullptr, Fd, dt, (T)0, (T)0);
   timing_end(c);
   c->launches += 7;
   return OSB_OK;
@@ -645,13 +689,13 @@ int filter_t(osb_ctx* c, Block& bl, double dt) {
   const T check = (T)bl.d.ducros_check;
   const long nf0 = (long)(k.n[0] + 1) * k.n[1] * k.n[2], nf1 = (long)k.n[0] * (k.n[1] + 1) * k.n[2],
              nf2 = (long)k.n[0] * k.n[1] * (k.n[2] + 1);
-  k_filter_flux<T, 0><<<grid_for(c, nf0, FT), FT, 0, c->stream>>>(k, sp, kappa, check, F[0], F[1], F[2], F[3], F[4]);
-  k_filter_flux<T, 1><<<grid_for(c, nf1, FT), FT, 0, c->stream>>>(k, sp, kappa, check, F[5], F[6], F[7], F[8], F[9]);
-  k_filter_flux<T, 2><<<grid_for(c, nf2, FT), FT, 0, c->stream>>>(k, sp, kappa, check, F[10], F[11], F[12], F[13],
+  k_filter_flux<T, 0><<<grid_for(c, (nf0 + FQ - 1) / FQ, FT), FT, 0, c->stream>>>(k, sp, kappa, check, F[0], F[1], F[2], F[3], F[4]);
+  k_filter_flux<T, 1><<<grid_for(c, (nf1 + FQ - 1) / FQ, FT), FT, 0, c->stream>>>(k, sp, kappa, check, F[5], F[6], F[7], F[8], F[9]);
+  k_filter_flux<T, 2><<<grid_for(c, (nf2 + FQ - 1) / FQ, FT), FT, 0, c->stream>>>(k, sp, kappa, check, F[10], F[11], F[12], F[13],
                                                                    F[14]);
   FilterFluxes<T> Fd;
   for (int a = 0; a < 15; ++a) Fd.f[a] = F[a];
-  k_filter_apply<T><<<grid_for(c, n, FT), FT, 0, c->stream>>>(k, kappa, Fd, dt, (T)bl.d.ducros_select);
+  k_filter_apply<T><<<grid_for(c, n, FT), FT, 0, c->stream>>>(k, kappa, Fd, dt, (T)bl.d.ducros_select, check);
   timing_end(c);
   c->launches += 8;
   return OSB_OK;

@@ -88,3 +88,25 @@ def test_sweeps_fp64_tiles(built_lib, oracle_lib, sizes, scheme, avg):
     for v in range(spec.nvars):
         scale = max(float(np.max(np.abs(ref[w][sl]))) for w in (mom if v in mom else (v,)))
         assert float(np.max(np.abs(got[v][sl] - ref[v][sl]))) < 1e-12 * scale, v
+
+
+# k_filter_flux lists the faces that are on among 512: none, some and all of them on; points selected
+# whose faces are off.  Tolerance 1e-10 as the other filter tests (WENO3-Z with an epsilon of 1e-40).
+@pytest.mark.parametrize("sizes", [(8, 8, 8), (7, 9, 11), (33, 16, 9)])
+@pytest.mark.parametrize("check,select", [(0.05, 0.05), (0.0, 0.0), (0.3, 0.01), (0.01, 0.3), (2.0, 0.0)])
+def test_filter_faces_fp64(built_lib, oracle_lib, sizes, check, select):
+    from opensbli_gb300.solver import Solver
+    spec, q = _block(sizes, abi.SCHEME_CENTRAL4, abi.VISC_SUTHERLAND, 14, minf=1.25)
+    spec.split_form, spec.filter = abi.SPLIT_KGP, abi.FILTER_WENO3
+    spec.ducros_check, spec.ducros_select = check, select
+    s = Solver([(spec, q)], precision="fp64", rk="ls3")
+    s.apply_bc()
+    s.step(2e-3, 1)
+    got = s.state(0)
+    s.close()
+    ob = harness.OracleBlocks([(spec, q)])
+    ob.apply_bc()
+    ob.step(abi.RK_LOW_STORAGE, problems.RK3_LS_A, problems.RK3_LS_B, 2e-3, 1)
+    sl = spec.interior()
+    errs = [harness.rel_err(got[v][sl], ob.q[0][v][sl]) for v in range(5)]
+    assert max(errs) < 1e-10, errs

@@ -4,8 +4,8 @@
 //                 state in shared memory (coalesced), then each lane sweeps one row
 //   k_flux_sweep  characteristic flux sweep along y or z: one thread per line segment,
 //                 coalesced along x, 6-point register window, one interface per step
-//   k_central3d   central 4th-order terms on a shared-memory tile: skew-symmetric convective
-//                 terms and/or viscous stress + heat flux
+//   k_central_wall  central 4th-order terms of blocks with walls (k_central of osb_central_tile.cuh
+//                 serves all others)
 //   k_rk          low-storage / SBLI RK update, counts non-finite values
 //   k_periodic / k_zero_grad / k_interface   boundary conditions
 //   k_reduce_*    FP64 diagnostics
@@ -270,7 +270,7 @@ struct RkFuse {
   float dt_h, dt_l;  // dt as a float-float pair
   float* qout[5];
   unsigned long long* bad;
-  unsigned long long* stall;  // bulk-staging waits that ran out (k_central3d BULK)
+  unsigned long long* stall;  // bulk-staging waits that ran out (k_central BULK)
 };
 
 // The increment dt * R of the FP32-residual path's RK update, from the float-float residual

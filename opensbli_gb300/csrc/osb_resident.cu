@@ -35,6 +35,7 @@ namespace {
 constexpr int RT = 256;        // most threads per CTA
 constexpr int RH = 3;          // stencil reach of the flux difference
 constexpr int RC = 16;         // most CTAs per cluster (8 where 16 are not to be had)
+constexpr size_t SMEM_MAX = 227 * 1024;  // shared memory of a CTA
 
 struct RkCoef {
   int kind, nst;
@@ -352,8 +353,9 @@ __global__ void __launch_bounds__(RT) k_resident_1d(const Resident1D* __restrict
 // (31 points), up to the largest cluster the GPU grants: below a warp an FP64 instruction costs the
 // same.  400 points: 16 CTAs of 25.  FP32: 125 points, four warps, which take as long as one (50
 // points, 20 steps: one CTA 0.160 ms, two 0.177; 400: 4 CTAs 0.17, 2 0.20, 1 0.30).  One CTA alone is no
-// cluster: a plain launch and CTA barriers.  Contexts of many blocks take smaller clusters (no fewer than
-// two CTAs where a block has more than 31 points: one holds about 1 600), enough to fill the SMs.
+// cluster: a plain launch and CTA barriers.  Contexts of many blocks take smaller clusters, enough to fill
+// the SMs: no fewer than two CTAs where a block has more than 31 points, and no larger shares than a
+// CTA's shared memory holds (FP64: 160 bytes a point, 1 448 points).
 template <typename T, int SCH, int AVG>
 int launch_resident(osb_ctx* c, const Resident1D* dev, int nblocks, int maxN, double dt, int nsteps) {
   const Block& f = c->blocks[0];
@@ -368,7 +370,8 @@ int launch_resident(osb_ctx* c, const Resident1D* dev, int nblocks, int maxN, do
   auto points = [&](int C) { return (maxN + C - 1) / C; };
   int C = 1;
   while (C < RC && points(C) > (sizeof(T) == 8 ? 31 : 125)) C *= 2;
-  while (C > 2 && (long)nblocks * (C / 2) >= 2L * c->sm_count) C /= 2;
+  auto fits = [&](int C) { return RLayout<T>::bytes(points(C)) <= SMEM_MAX; };
+  while (C > 2 && (long)nblocks * (C / 2) >= 2L * c->sm_count && fits(C / 2)) C /= 2;
   auto kern = k_resident_1d<T, SCH, AVG>;
   if (C > 8) OSB_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
   cudaLaunchConfig_t cfg{};

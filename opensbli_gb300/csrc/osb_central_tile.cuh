@@ -34,7 +34,7 @@
 // plane's arithmetic; through shared memory a plane ahead (cp.async) they gained nothing (viscous) or
 // lost 20 % (KGP: one more CTA's worth of shared memory).  256^3 viscous + update 0.92 -> 0.82 ms per
 // stage (240 bytes per point, 4.9 TB/s), 131 x 97 x 110 0.109 -> 0.096, 64^3 Feiereisen + update 27 ->
-// 22 us, KGP 128^3 0.168 -> 0.133 ms.
+// 22 us, KGP 128^3 0.168 -> 0.134 ms.
 //
 // BULK (FP32 state only): the raw planes come in through the bulk-copy (TMA) engine instead --
 // one cp.async.bulk per staged row and variable into a two-slot raw buffer in shared memory,
@@ -52,13 +52,13 @@ constexpr int CTPP = (CTPL + CTT - 1) / CTT;   // staged points per thread and p
 constexpr int CTRAW = 2 * 5 * CTSY * CRW;      // floats of the two raw plane slots (BULK)
 
 // Staged fields: velocity; VISC: temperature (and viscosity unless constant); CONV: momentum, then
-// Feiereisen E / rho, p + E / 2 and 2 p, or KGP H, rho and p (with viscous terms p is rho T over a
-// constant, and two CTAs' rings fit an SM next to the update's buffer).
+// Feiereisen E / rho, p + E / 2 and 2 p, or KGP H, rho and p (p itself also with viscous terms: rho T
+// would round a uniform pressure differently at every density).  FP32: two CTAs' rings fit an SM.
 template <int CONV, int VISC>
 struct CtFields {
   static constexpr int U = 0, TT = 3, MU = 4;
   static constexpr int M = 3 + (VISC ? (VISC == 1 ? 2 : 1) : 0), EE = M + 3, HH = M + 4, P = M + 5;
-  static constexpr int N = CONV ? (CONV == 2 && VISC ? M + 5 : M + 6) : M;
+  static constexpr int N = CONV ? M + 6 : M;
 };
 template <typename T, int CONV, int VISC, bool BULK>
 constexpr size_t ct_smem() {
@@ -101,7 +101,7 @@ __global__ void __launch_bounds__(CTT, ct_ctas<T, CONV, VISC, BULK>())
   const int x0 = blockIdx.x * CX, y0 = blockIdx.y * CTY;
   const int zb = blockIdx.z * czc, ze = min(b.n[2], zb + czc);
   const T gm = cpar<T>(cp.gama, cp.gama_f), g1 = gm - L_(1.0);
-  const T M2g = cpar<T>(cp.M2, cp.M2_f) * gm, iM2g = recip(M2g);
+  const T M2g = cpar<T>(cp.M2, cp.M2_f) * gm;
   const T mu_pw = cpar<T>(cp.mu_pow, cp.mu_pow_f);
   T qv[CTPP][5];
   // WRAP: the staged points' images in x and y, the same for every plane
@@ -152,7 +152,7 @@ __global__ void __launch_bounds__(CTT, ct_ctas<T, CONV, VISC, BULK>())
         at[(Fd::M + 0) * FS] = m0;
         at[(Fd::M + 1) * FS] = m1;
         at[(Fd::M + 2) * FS] = m2;
-        if (CONV == 1 || !VISC) at[Fd::P * FS] = CONV == 1 ? L_(2.0) * p : p;
+        at[Fd::P * FS] = CONV == 1 ? L_(2.0) * p : p;
         at[Fd::EE * FS] = CONV == 1 ? E * ir : (E + p) * ir;
         at[Fd::HH * FS] = CONV == 1 ? fmat(L_(0.5), E, p) : rho;
       }
@@ -464,21 +464,7 @@ __global__ void __launch_bounds__(CTT, ct_ctas<T, CONV, VISC, BULK>())
       if (CONV == 2) {
         racc[0] = -L_(0.5) * cr;
 #pragma unroll
-        for (int i = 0; i < 3; ++i) {
-          T dp0;
-          if (VISC) {  // p = rho T / (gama M^2)
-            T pr[4];
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-              const int m = k < 2 ? k - 2 : k - 1;
-              pr[k] = F(Fd::HH, i, m) * F(Fd::TT, i, m);
-            }
-            dp0 = d1(i, pr[0], pr[1], pr[2], pr[3]) * iM2g;
-          } else {
-            dp0 = D1(Fd::P, i);
-          }
-          racc[1 + i] = -fmat(L_(0.25), cm[i], dp0);
-        }
+        for (int i = 0; i < 3; ++i) racc[1 + i] = -fmat(L_(0.25), cm[i], D1(Fd::P, i));
         racc[4] = -L_(0.25) * ce;
       }
       if (VISC) {

@@ -735,7 +735,10 @@ __device__ __forceinline__ float2 rcp2(float2 a) { return f2(rcp_approx(a.x), rc
 __device__ __forceinline__ float2 abs2(float2 a) { return f2(fabsf(a.x), fabsf(a.y)); }
 
 // recon5 (FP32 form: see its epsilon) of two waves at once, on the differences of the stencil values.
-// s2: the square of the waves' scale (ReconEps), which the absolute epsilon of WENO5-JS takes.
+// s2: the square of the waves' scale (ReconEps), which the absolute epsilon of WENO5-JS takes.  The floor
+// under every epsilon, 4e-36, only keeps a wave without differences off 0/0 (FP32 still holds its
+// reciprocal): these waves carry the density, and at 4e-30 it swamped the indicators of a thin gas
+// (below about 1e-13).
 template <int SCH>
 __device__ __forceinline__ float2 recon5_x2(float2 fm2, float2 fm1, float2 f0, float2 fp1, float2 fp2, float eps_rel,
                                             float ct, float2 s2) {
@@ -746,10 +749,10 @@ __device__ __forceinline__ float2 recon5_x2(float2 fm2, float2 fm1, float2 f0, f
   // four times epsilon: relative to the stencil's mean square, or WENO5-JS's constant
   float2 e4;
   if (SCH == SCH_WENO5_JS) {
-    e4 = mul2(f2(4.0e-6f), s2);
+    e4 = fma2(f2(4.0e-6f), s2, f2(4e-36f));
   } else {
     const float2 ss = fma2(fp2, fp2, fma2(fp1, fp1, fma2(f0, f0, fma2(fm1, fm1, mul2(fm2, fm2)))));
-    e4 = fma2(f2(0.8f * eps_rel), ss, f2(4e-30f));
+    e4 = fma2(f2(0.8f * eps_rel), ss, f2(4e-36f));
   }
   const float2 k = f2((float)(13.0 / 3.0));
   const float2 u0 = fma2(mul2(k, c0), c0, fma2(s0, s0, e4));

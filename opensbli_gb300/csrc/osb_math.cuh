@@ -749,7 +749,7 @@ __device__ __forceinline__ float2 recon5_x2(float2 fm2, float2 fm1, float2 f0, f
   // four times epsilon: relative to the stencil's mean square, or WENO5-JS's constant
   float2 e4;
   if (SCH == SCH_WENO5_JS) {
-    e4 = fma2(f2(4.0e-6f), s2, f2(4e-36f));
+    e4 = f2(4.0e-6f * s2.x + 4e-36f, 4.0e-6f * s2.y + 4e-36f);  // a constant where s2 is one
   } else {
     const float2 ss = fma2(fp2, fp2, fma2(fp1, fp1, fma2(f0, f0, fma2(fm1, fm1, mul2(fm2, fm2)))));
     e4 = fma2(f2(0.8f * eps_rel), ss, f2(4e-36f));

@@ -8,7 +8,8 @@
 // sweeps), the residual and the RK update (rk_LS.py:204-215 / rk_sbli.py:138-154).  A CTA owns a
 // run of points; after an update it writes its outer three points into its neighbours' shared
 // memory, and one cluster barrier ends the stage.  One cluster per block: blocks of one context
-// advance independently (no interfaces).  Both precisions.
+// advance independently (no interfaces).  Both precisions; FP32 blocks of a few hundred points, and
+// contexts with more of them than the chip has room for clusters, take one CTA each (k_resident_cta).
 //
 // FP64 is bound by the FP64 pipe (one warp instruction per 16 cycles and SM), so the points go to as
 // many SMs as still get a full warp of interfaces: one CTA took 61 us a stage for 400 points (100 us
@@ -349,11 +350,136 @@ __global__ void __launch_bounds__(RT) k_resident_1d(const Resident1D* __restrict
   if (nb) atomicAdd(bad, nb);
 }
 
+#ifdef OSB_RESIDENT_F32
+// Boundary treatment of one 1D block held in shared memory (x fastest, halo h): periodic,
+// zero-gradient and extrapolation as k_periodic / k_zero_grad / k_extrap; side 0 then side 1.
+__device__ void bc_1d(double* q, int E, int h, int N, const Resident1D& r) {
+  const int t = threadIdx.x;
+  if (r.bc[0] == OSB_BC_PERIODIC) {
+    // both sides in one pass (they read the interior only): [0, d) -> [N, N+d), [N-d, N) -> [-d, 0)
+    const int d0 = r.depth[0], d1 = r.depth[1];
+    for (int u = t; u < 3 * (d0 + d1); u += blockDim.x) {
+      const int v = u / (d0 + d1), m = u % (d0 + d1);
+      double* f = q + v * E + h;
+      if (m < d0) f[N + m] = f[m];
+      else f[-d1 + (m - d0)] = f[N - d1 + (m - d0)];
+    }
+    return;
+  }
+  if (t < 6) {
+    const int side = t / 3, v = t % 3;
+    double* f = q + v * E + h;
+    const int kind = r.bc[side], depth = r.depth[side];
+    const int id = side == 0 ? 0 : N - 1;
+    const int s = side == 0 ? 1 : -1;  // inward step
+    if (kind == OSB_BC_ZERO_GRAD) {
+      f[id] = f[id + s];
+      for (int m = 1; m <= depth; ++m) f[id - m * s] = f[id + m * s];
+    } else if (kind == OSB_BC_EXTRAP0) {
+      f[id] = f[id + s];
+      for (int m = 1; m <= depth; ++m) f[id - m * s] = f[id + s];
+    } else if (kind == OSB_BC_EXTRAP1) {
+      for (int m = 1; m <= depth; ++m) f[id - m * s] = -f[id - (m - 2) * s] + 2.0 * f[id - (m - 1) * s];
+    }
+  }
+}
+
+// FP32 blocks that one CTA runs alone, halos and an FP32 copy of the state in its shared memory: every
+// interface forms its six points' primitives itself, which costs less than staging them where the
+// chain of a stage counts and not the arithmetic (see launch_resident for both sides' times).
+template <int SCH, int AVG>
+__global__ void __launch_bounds__(RT) k_resident_cta(const Resident1D* __restrict__ blocks, SchemeParams spd, RkCoef rk,
+                                                     double dt, int nsteps, unsigned long long* bad) {
+  const Resident1D r = blocks[blockIdx.x];
+  const BlockK& b = r.k;
+  const SP<float> sp(spd);
+  extern __shared__ __align__(16) unsigned char osb_smem[];
+  const int N = b.n[0], h = b.off0, E = b.alloc;
+  double* q = reinterpret_cast<double*>(osb_smem);   // [3][E]
+  double* o = q + 3 * E;                              // [3][E]
+  float* F = reinterpret_cast<float*>(o + 3 * E);     // [3][E]: flux at the right face of point i
+  float* qf = F + 3 * E;                              // [3][E]: FP32 copy of the state
+  for (int u = threadIdx.x; u < 3 * E; u += blockDim.x) {
+    q[u] = b.q[u / E][u % E];
+    o[u] = b.rk[u / E][u % E];
+    qf[u] = d2f_rn(q[u]);
+  }
+  const float invd_f = (float)b.invd[0];
+  const float dt_h = (float)dt, dt_l = (float)(dt - (double)dt_h);
+  for (int step = 0; step < nsteps; ++step) {
+    __syncthreads();     // the previous stage's update is complete
+    if (rk.kind == 1) {  // SBLI RK3 saves the state at the start of the step
+      for (int u = threadIdx.x; u < 3 * N; u += blockDim.x) o[(u / N) * E + h + u % N] = q[(u / N) * E + h + u % N];
+    }
+    for (int s = 0; s < rk.nst; ++s) {
+      __syncthreads();
+      bc_1d(q, E, h, N, r);
+      __syncthreads();
+      // the boundary treatment changed the halos and at most the end points: refresh their copy
+      for (int u = threadIdx.x; u < 3 * 2 * (h + 2); u += blockDim.x) {
+        const int v = u / (2 * (h + 2)), m = u % (2 * (h + 2));
+        const int i = m < h + 2 ? m - h : N - 2 + (m - (h + 2));
+        qf[v * E + h + i] = d2f_rn(q[v * E + h + i]);
+      }
+      __syncthreads();
+      for (int i = (int)threadIdx.x - 1; i < N; i += blockDim.x) {
+        Pt<float, 1> w[6];
+#pragma unroll
+        for (int m = 0; m < 6; ++m) {
+#pragma unroll
+          for (int v = 0; v < 3; ++v) w[m].q[v] = qf[v * E + h + i - 2 + m];
+          make_pt<float, 1>(w[m], sp.gama);
+        }
+        float fh[3];
+        char_flux<float, 1, SCH, AVG>(w, sp, fh);
+#pragma unroll
+        for (int v = 0; v < 3; ++v) F[v * E + h + i] = fh[v];
+      }
+      __syncthreads();
+      const double A = rk.A[s], B = rk.B[s];
+      const bool a_zero = rk.kind == 0 && A == 0.0;
+      for (int i = threadIdx.x; i < N; i += blockDim.x) {
+#pragma unroll
+        for (int v = 0; v < 3; ++v) {
+          const int id = v * E + h + i;
+          double ov = o[id], qv = q[id];
+          float p, pe;
+          ff_flux_diff(F[id], F[id - 1], invd_f, p, pe);
+          const float hh = __fadd_rn(p, pe);
+          const float ll = __fsub_rn(pe, __fsub_rn(hh, p));
+          const double x = dt_residual(hh, ll, dt_h, dt_l);  // as rk_point
+          if (rk.kind == 0) {
+            ov = a_zero ? x : __fma_rn(A, ov, x);
+            qv = __fma_rn(B, ov, qv);
+          } else {
+            qv = __fma_rn(A, x, ov);
+            ov = __fma_rn(B, x, ov);
+          }
+          qf[id] = d2f_rn(qv);
+          o[id] = ov;
+          q[id] = qv;
+        }
+      }
+    }
+  }
+  __syncthreads();
+  bc_1d(q, E, h, N, r);  // the halos a caller observes after the call
+  __syncthreads();
+  unsigned long long nb = 0;
+  for (int u = threadIdx.x; u < 3 * E; u += blockDim.x) {
+    b.q[u / E][u % E] = q[u];
+    b.rk[u / E][u % E] = o[u];
+    const int i = u % E - h;
+    if (i >= 0 && i < N && !isfinite(q[u])) ++nb;
+  }
+  if (nb) atomicAdd(bad, nb);
+}
+#endif
+
 // Points are split over the smallest power of two of CTAs that leaves each a warp of interfaces
 // (31 points), up to the largest cluster the GPU grants: below a warp an FP64 instruction costs the
-// same.  400 points: 16 CTAs of 25.  FP32: 125 points, four warps, which take as long as one (50
-// points, 20 steps: one CTA 0.160 ms, two 0.177; 400: 4 CTAs 0.17, 2 0.20, 1 0.30).  One CTA alone is no
-// cluster: a plain launch and CTA barriers.  Contexts of many blocks take smaller clusters, enough to fill
+// same.  400 points: 16 CTAs of 25.  FP32: 125 points, four warps, which take as long as one (400
+// points, 20 steps: 4 CTAs 0.17 ms, 2 0.20).  One CTA alone is no cluster: a plain launch and CTA barriers.  Contexts of many blocks take smaller clusters, enough to fill
 // the SMs: no fewer than two CTAs where a block has more than 31 points, and no larger shares than a
 // CTA's shared memory holds (FP64: 160 bytes a point, 1 448 points).
 template <typename T, int SCH, int AVG>
@@ -379,7 +505,7 @@ int launch_resident(osb_ctx* c, const Resident1D* dev, int nblocks, int maxN, do
   at.id = cudaLaunchAttributeClusterDimension;
   cfg.attrs = &at;
   cfg.stream = c->stream;
-  int most = 0;
+  int most = 0, granted = 0;  // points of the largest share; clusters of this shape that run at once
   for (;; C /= 2) {
     most = std::max(points(C), 4 * RH);  // a smaller block's share: below 2 (2 RH) points each
     const size_t smem = RLayout<T>::bytes(most);
@@ -391,11 +517,45 @@ int launch_resident(osb_ctx* c, const Resident1D* dev, int nblocks, int maxN, do
     const int W = (most + 32) / 32 * 32;
     cfg.blockDim = dim3((unsigned)std::min(RT, sizeof(T) == 8 ? 3 * W : (most + 2 * RH + 31) / 32 * 32));
     cfg.dynamicSmemBytes = smem;
-    if (C <= 8) break;  // a portable cluster size
-    int granted = 0;
+    granted = nblocks;
+    if (C <= 8 && (sizeof(T) == 8 || (long)nblocks * C <= 2L * c->sm_count)) break;
     if (cudaOccupancyMaxActiveClusters(&granted, kern, &cfg) == cudaSuccess && granted > 0) break;
     cudaGetLastError();
+    granted = 0;
+    if (C <= 8) break;  // a portable cluster size
   }
+#ifdef OSB_RESIDENT_F32
+  // One CTA per block (k_resident_cta) or the cluster, 20 steps, CTA and cluster:
+  //  - up to 244 points (two CTAs of the cluster) the CTA's chain is the shorter one: 6 points 0.113 and 0.138 ms,
+  //    100 points 0.118 and 0.133, 200 points 0.143 and 0.157; 255 points 0.146 and 0.125, but from half as many
+  //    blocks as SMs on the CTA again (100 blocks 0.151 and 0.173);
+  //  - many larger blocks, of similar sizes, whose clusters do not all run at once: 300 points x 256 0.296 and
+  //    0.463, 400 x 150 0.249 and 0.382, 600 x 130 0.323 and 0.450, 1000 x 220 0.644 and 0.760; where they do,
+  //    the cluster: 600 x 100 0.313 and 0.231, 300 x 220 0.297 and 0.245; a few blocks too (1500 x 40 0.613 and
+  //    0.406).  The CTA has to leave room for a second one on its SM (2 000 points x 304 1.61 and 1.41).
+  // The CTA has a thread per interface, and 64 at least while the blocks leave SMs with room (6 points: 32
+  // threads 0.122, 64 0.113; 1 500 blocks 0.193 and 0.309).
+  long alloc = 0, sum = 0;
+  for (const auto& bl : c->blocks) {
+    alloc = std::max(alloc, bl.k.alloc);
+    sum += bl.k.n[0];
+  }
+  const size_t cta_smem = (size_t)3 * alloc * (2 * sizeof(double) + 2 * sizeof(float));
+  const bool waves = granted < nblocks && 5 * nblocks >= 3 * c->sm_count && 2 * sum > (long)maxN * nblocks &&
+                     2 * (cta_smem + 1024) <= 228 * 1024;
+  if (maxN <= 244 || (maxN <= 255 && 2 * nblocks >= c->sm_count) || waves) {
+    auto cta = k_resident_cta<SCH, AVG>;
+    if (cta_smem > 48 * 1024)
+      OSB_CK(cudaFuncSetAttribute(cta, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cta_smem));
+    const int threads = std::max(nblocks <= 2 * c->sm_count ? 64 : 32, std::min(RT, (maxN + 32) / 32 * 32));
+    timing_begin(c, FAM_PERSISTENT);
+    cta<<<nblocks, threads, cta_smem, c->stream>>>(dev, sp, rk, dt, nsteps, c->bad);
+    timing_end(c);
+    c->launches++;
+    OSB_CK(cudaGetLastError());
+    return OSB_OK;
+  }
+#endif
   timing_begin(c, FAM_PERSISTENT);
   OSB_CK(cudaLaunchKernelEx(&cfg, kern, dev, sp, rk, dt, nsteps, most, c->bad));
   timing_end(c);

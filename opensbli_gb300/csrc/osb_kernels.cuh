@@ -521,8 +521,15 @@ __global__ void __launch_bounds__(SWEEP_THREADS, sizeof(T) == 4 ? 3 : 1)
 constexpr int XCH = 4, XRING = 2, XCOLS = XCH * XRING, XPITCH = XCOLS + 1, XOUT = 8, XOPITCH = XOUT + 1;
 // FP32: six CTAs of two warps per SM, 168 registers (256^3 TENO5: 0.61 ms; 0.76 with eight CTAs at
 // 128; 0.86 before the packed flux).  Curvilinear: four CTAs, 255 registers (4-block case 2.8 ms a
-// step; 4.8 with six).
+// step; 4.8 with six), but the compiler's own choice for TENO on 2D blocks (TENO5, 4 steps of 64^2 / 400^2 /
+// 1000^2: 0.64 / 0.70 / 1.77 ms; with four CTAs 0.68 / 0.75 / 1.79).
 constexpr int XWARPS = 2;
+template <typename T, int ND, int SCH, bool CURV>
+constexpr int x_ctas() {
+  if (sizeof(T) == 8) return 1;
+  if (CURV) return generated_order<ND, SCH>() ? 0 : 4;
+  return 6;
+}
 
 template <typename T, int NF, int NO>
 struct XTile {
@@ -532,8 +539,8 @@ struct XTile {
 };
 
 template <typename T, int ND, int SCH, int AVG, bool CURV, int FLX = 0>
-__global__ void __launch_bounds__(32 * XWARPS, sizeof(T) == 4 ? (CURV ? 4 : 6) : 1) k_flux_x(BlockK b, SchemeParams spd, int first, int xseg,
-                                                         const int* __restrict__ xrows) {
+__global__ void __launch_bounds__(32 * XWARPS, x_ctas<T, ND, SCH, CURV>())
+    k_flux_x(BlockK b, SchemeParams spd, int first, int xseg, const int* __restrict__ xrows) {
   constexpr int NV = ND + 2;
   constexpr int NF = SweepFields<ND, CURV>::N;
   constexpr int NO = CURV ? NV + 1 : NV;  // curvilinear: the point's 1 / (dx J) rides along

@@ -182,7 +182,7 @@ static __device__ const double teno5_rows[8][4] = {
 #undef OSB_TENO5_ROW
 
 // Blocks whose flux keeps the generated order of operations (projections, primitives, divisions and
-// indicators; recon5_ieee says why), in both precisions.
+// indicators) in both precisions: recon5_ieee says why these and what the others differ by.
 template <int ND, int SCH>
 __host__ __device__ constexpr bool generated_order() {
   return ND <= 2 && (SCH == SCH_TENO5 || SCH == SCH_TENO6);
@@ -190,13 +190,18 @@ __host__ __device__ constexpr bool generated_order() {
 
 // Fifth-order reconstruction in the generated order with IEEE divisions, FP64.  It serves
 //   - values beyond the range of recon5_f64's common denominator,
-//   - TENO5 on 1D and 2D blocks (generated_order; TENO6 keeps the order too).  A front in exactly uniform gas is symmetric
-//     at first, so the outer indicators of a five-point window tie while the middle one is zero to
+//   - TENO5 on 1D and 2D blocks (generated_order; TENO6 keeps the order too).  Beside a front in exactly
+//     uniform gas the outer indicators of a five-point window can tie while the middle one is zero to
 //     rounding: tau is then the rounding of b0 - b2, and whether it is exactly zero decides if TENO5
-//     keeps the outer stencils.  Another order of the same operations moves a shock tube by 1e-7
-//     and a shear layer by 1e-5 of their size within ten steps (the WENO weights: below 1e-14).  3D
-//     blocks, with smooth fields in all directions, take recon5_f64 (a step of the 128^3 TENO5 vortex in
-//     the generated order 63 ms, with it 17).
+//     keeps the outer stencils.  No order of the operations decides such a tie better than another: on
+//     shear layers extruded to 3D, 9 steps, the generated order lies 3e-6 .. 3e-4 of the largest value
+//     from plain IEEE arithmetic (median over 12 layers at three sizes), recon5_f64 5e-7 .. 6e-5; FP32 1e-3
+//     and 1e-3.  1D and 2D blocks keep the order of the generated solver, so that their results are
+//     the ones they always were; 3D blocks take recon5_f64 (a step of the 128^3 TENO5 vortex in the
+//     generated order 68 ms, with it 17).
+// WENO5-Z has such ties at zero-gradient ends: the mirrored window (x, y, y, y, x) has b0 = b2 and b1 = 0.  The
+// differences make tau exactly zero there and the weights linear; the generated order does in 37 - 49 % of
+// such windows and takes stencil [-1, 0, 1] alone in the others.
 template <int SCH>
 __device__ __forceinline__ double recon5_ieee(double fm2, double fm1, double f0, double fp1, double fp2, double eps,
                                               double ct) {

@@ -7,6 +7,7 @@ oracle/ops_compat.h), interior points only, FP64, as a compressed .npz:
 
     python tests/golden/make_golden.py            # all cases
     python tests/golden/make_golden.py tvd        # the TVD-filtered TGV
+    python tests/golden/make_golden.py teno5_ties # on a GPU: see make_teno5_ties
 """
 import os
 import subprocess
@@ -21,6 +22,7 @@ sys.path.insert(0, os.path.join(ROOT, "oracle"))
 
 import harness  # noqa: E402
 from opensbli_gb300 import abi, problems  # noqa: E402
+from opensbli_gb300.spec import BlockSpec  # noqa: E402
 
 
 def perturb(q, amp, seed):
@@ -235,7 +237,38 @@ def make_mb2_flip(sizes=(24, 20), counts=(1, 3, 30), dt=5e-4, pert=(1e-3, 31)):
     print("wrote", name)
 
 
+def make_teno5_ties():
+    """The states of teno5_ties.npz again from the file's own initial states, on a GPU: nine steps of
+    this library's per-block path.  Unlike the other golden files it records the order of operations of
+    1D and 2D TENO5 blocks as the GPU build rounds it, which decides tied stencils; the CPU test of the
+    file says how near the oracle is."""
+    from opensbli_gb300.solver import Solver
+    path = os.path.join(HERE, "teno5_ties.npz")
+    out = dict(np.load(path))
+    for name in ("sod", "kh", "kh_fp32"):
+        n = out[name + "_q0"].shape[1:]
+        common = dict(scheme=abi.SCHEME_TENO5, gama=1.4, eps=1e-40)
+        if name == "sod":
+            z = abi.BC_ZERO_GRAD
+            size = (n[0] - 10,)
+            spec = BlockSpec(ndim=1, size=size, bc=[[z, z]], bc_depth=[[4, 4]], delta=[1.0 / (size[0] - 1)],
+                             averaging=abi.AVG_SIMPLE, **common)
+        else:
+            size = (n[1] - 10, n[0] - 10)
+            spec = BlockSpec(ndim=2, size=size, delta=(1.0 / size[0], 1.0 / size[1]), averaging=abi.AVG_ROE, **common)
+        s = Solver([(spec, list(out[name + "_q0"]))], precision="fp32" if name == "kh_fp32" else "fp64", rk="ls3")
+        s.set_schedule(mode=abi.SCHED_PER_BLOCK)
+        s.step(float(out[name + "_dt"]), 9)
+        out[name + "_q"] = np.stack(s.state(0))
+        s.close()
+    np.savez_compressed(path, **out)
+    print("wrote teno5_ties")
+
+
 def main():
+    if sys.argv[1:] == ["teno5_ties"]:
+        make_teno5_ties()
+        return
     if sys.argv[1:] == ["mb2_flip"]:
         make_mb2_flip()
         return

@@ -58,6 +58,7 @@ int launch_tile(osb_ctx* c, Block& bl, const SchemeParams& sp) {
   const long lines = (long)k.n[0] * k.n[1] * k.n[2] / k.n[D];
   const int parts = (k.n[D] + Tl::NI - 2) / (Tl::NI - 1), pts = (k.n[D] + parts - 1) / parts;
   const long gx = (lines + Tl::NC - 1) / Tl::NC;
+  // more rows than the line sweeps take are refused here too
   if (parts > 65535 || (D > 0 && lines / k.n[0] > 65535)) return fail(OSB_ENOTSUP, "block too large for the sweep grid");
   timing_begin(c, D == 0 ? FAM_FLUX_X : D == 1 ? FAM_FLUX_Y : FAM_FLUX_Z);
   kern<<<dim3((unsigned)gx, (unsigned)parts), F64T, smem, c->stream>>>(k, sp, pts, D == 0 ? 1 : 0);

@@ -182,7 +182,7 @@ inline int wave_chunks(int n, long ctas_per_chunk, long slots, double overhead, 
 // Grid size of a grid-stride launch over n items: enough CTAs to cover them, at most 8 per SM.
 int grid_for(osb_ctx* c, long n, int threads);
 
-// Whole osb_step calls of small 1D blocks in one launch, one CTA per block (osb_resident.cu).
+// Whole osb_step calls of small 1D blocks in one launch, a cluster of CTAs or one CTA per block (osb_resident.cu).
 bool resident_eligible(const osb_ctx* c);
 int resident_step(osb_ctx* c, double dt, int nsteps);
 int resident_f64(osb_ctx* c, double dt, int nsteps);

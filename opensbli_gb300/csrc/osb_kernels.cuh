@@ -671,7 +671,7 @@ struct CentralParams {
   float gama_f, M2_f, mu_c_f, invRe_f, kheat_f;
   double invd[3], inv2d[3];
   float invd_f[3], inv2d_f[3];
-  // isothermal-wall y faces (WALL kernels): low / high face present, and the one-sided
+  // wall y faces (k_central_wall): low / high face present, and the one-sided
   // closures of the first (rows 0..3, six points from m - r) and second (rows 0..1, five
   // points) derivatives next to a wall (Carpenter_scheme.py)
   int wall_lo, wall_hi;
@@ -751,14 +751,12 @@ struct WallFields {
 
 template <typename T, int VISC, bool FUSE>
 __global__ void __launch_bounds__(CX * CWY) k_central_wall(BlockK b, CentralParams cp, int first, int czc, RkFuse rf) {
-  constexpr int CY = CWY;
-  constexpr bool WALL = true;
   using Fd = WallFields;
   constexpr int FS = CRING * CPL;  // field stride in shared memory
   extern __shared__ __align__(16) unsigned char osb_smem[];
   T* sm = reinterpret_cast<T*>(osb_smem);
   const int tx = threadIdx.x % CX, ty = threadIdx.x / CX;
-  const int x0 = blockIdx.x * CX, y0 = blockIdx.y * CY;
+  const int x0 = blockIdx.x * CX, y0 = blockIdx.y * CWY;
   const int zb = blockIdx.z * czc, ze = min(b.n[2], zb + czc);
   const T gm = cpar<T>(cp.gama, cp.gama_f);
   const T M2 = cpar<T>(cp.M2, cp.M2_f);
@@ -771,7 +769,7 @@ __global__ void __launch_bounds__(CX * CWY) k_central_wall(BlockK b, CentralPara
   auto load_plane = [&](int gz) {
 #pragma unroll
     for (int u = 0; u < CPP; ++u) {
-      const int idx = threadIdx.x + u * CX * CY;
+      const int idx = threadIdx.x + u * CX * CWY;
       const int gx = x0 - CH + idx % CSX, gy = y0 - CHY + idx / CSX;
       if (idx < CPL && gx <= b.n[0] + CH && gy <= b.n[1] + CHY) {
         const int id = lin(b, gx, gy, gz);
@@ -784,7 +782,7 @@ __global__ void __launch_bounds__(CX * CWY) k_central_wall(BlockK b, CentralPara
   auto store_plane = [&](int slot) {
 #pragma unroll
     for (int u = 0; u < CPP; ++u) {
-      const int idx = threadIdx.x + u * CX * CY;
+      const int idx = threadIdx.x + u * CX * CWY;
       const int gx = x0 - CH + idx % CSX, gy = y0 - CHY + idx / CSX;
       if (!(idx < CPL && gx <= b.n[0] + CH && gy <= b.n[1] + CHY)) continue;
       const int at = slot * CPL + idx;
@@ -817,53 +815,49 @@ __global__ void __launch_bounds__(CX * CWY) k_central_wall(BlockK b, CentralPara
   const T id0 = cpar<T>(cp.invd[0], cp.invd_f[0]), id2 = cpar<T>(cp.invd[2], cp.invd_f[2]);
   const T jd0 = cpar<T>(cp.inv2d[0], cp.inv2d_f[0]), jd2 = cpar<T>(cp.inv2d[2], cp.inv2d_f[2]);
   T id1 = cpar<T>(cp.invd[1], cp.invd_f[1]), jd1 = cpar<T>(cp.inv2d[1], cp.inv2d_f[1]);
-  // WALL on a stretched y grid (metric.py:199-240, SD111 the only second-derivative metric):
+  // stretched y grid (metric.py:199-240, SD111 the only second-derivative metric):
   // every y derivative of this thread's row takes D11 (d/dx_1 = D11 d/dxi_1, so 1/Delta_1 and
   // 1/Delta_1^2 scale by D11 and D11^2), and the second ones add D11 SD111 d/dxi_1 = SD111 times
   // the scaled first derivative
   T sdy = L_(0.0);
-  if constexpr (WALL) {
-    if (b.ys[0] && gy < b.n[1]) {
-      const T d11 = ystr<T>(b, 0, gy);
-      id1 = id1 * d11;
-      jd1 = jd1 * (d11 * d11);
-      sdy = ystr<T>(b, 1, gy);
-    }
+  if (b.ys[0] && gy < b.n[1]) {
+    const T d11 = ystr<T>(b, 0, gy);
+    id1 = id1 * d11;
+    jd1 = jd1 * (d11 * d11);
+    sdy = ystr<T>(b, 1, gy);
   }
   // offsets are written as linear offsets of a virtual (x, y, z) tile with z stride CPL and
   // decoded into (plane, in-plane) parts; they are compile-time constants after unrolling
   const int sx = 1, sy = CSX, sz = CPL;
   const int cxy = (ty + CHY) * CSX + (tx + CH);
-  // WALL: the closure rows of this thread's point (wr1: first derivatives, rows 0..3 from a
+  // the closure rows of this thread's point (wr1: first derivatives, rows 0..3 from a
   // wall; wr2: second derivatives, rows 0..1; -1 the central rule), its weights with the sign of
   // the face applied, and the y offsets m -> yb + ys m of the stencil points
   int wr1 = -1, wr2 = -1, yb1 = 0, ys1 = 1, yb2 = 0, ys2 = 1;
   T cw1[6], cw2[5];
-  if constexpr (WALL) {
-    const int ny = b.n[1];
-    if (gy < ny) {
-      if (cp.wall_lo && gy < 4) wr1 = gy;
-      else if (cp.wall_hi && gy > ny - 5) wr1 = 4 + (ny - 1 - gy);
-      if (cp.wall_lo && gy < 2) wr2 = gy;
-      else if (cp.wall_hi && gy > ny - 3) wr2 = 4 + (ny - 1 - gy);
-    }
-    const int r1 = wr1 & 3, r2 = wr2 & 1;
-    const bool hi1 = wr1 >= 4, hi2 = wr2 >= 4;
-    yb1 = hi1 ? r1 : -r1;
-    ys1 = hi1 ? -1 : 1;
-    yb2 = hi2 ? r2 : -r2;
-    ys2 = hi2 ? -1 : 1;
-#pragma unroll
-    for (int m = 0; m < 6; ++m) {
-      const T c = r1 == 0 ? cpar<T>(cp.c1[0][m], cp.c1f[0][m])
-                  : r1 == 1 ? cpar<T>(cp.c1[1][m], cp.c1f[1][m])
-                  : r1 == 2 ? cpar<T>(cp.c1[2][m], cp.c1f[2][m])
-                            : cpar<T>(cp.c1[3][m], cp.c1f[3][m]);
-      cw1[m] = hi1 ? -c : c;
-    }
-#pragma unroll
-    for (int m = 0; m < 5; ++m) cw2[m] = r2 == 0 ? cpar<T>(cp.c2[0][m], cp.c2f[0][m]) : cpar<T>(cp.c2[1][m], cp.c2f[1][m]);
+  const int ny = b.n[1];
+  if (gy < ny) {
+    if (cp.wall_lo && gy < 4) wr1 = gy;
+    else if (cp.wall_hi && gy > ny - 5) wr1 = 4 + (ny - 1 - gy);
+    if (cp.wall_lo && gy < 2) wr2 = gy;
+    else if (cp.wall_hi && gy > ny - 3) wr2 = 4 + (ny - 1 - gy);
   }
+  const int r1 = wr1 & 3, r2 = wr2 & 1;
+  const bool hi1 = wr1 >= 4, hi2 = wr2 >= 4;
+  yb1 = hi1 ? r1 : -r1;
+  ys1 = hi1 ? -1 : 1;
+  yb2 = hi2 ? r2 : -r2;
+  ys2 = hi2 ? -1 : 1;
+#pragma unroll
+  for (int m = 0; m < 6; ++m) {
+    const T c = r1 == 0 ? cpar<T>(cp.c1[0][m], cp.c1f[0][m])
+                : r1 == 1 ? cpar<T>(cp.c1[1][m], cp.c1f[1][m])
+                : r1 == 2 ? cpar<T>(cp.c1[2][m], cp.c1f[2][m])
+                          : cpar<T>(cp.c1[3][m], cp.c1f[3][m]);
+    cw1[m] = hi1 ? -c : c;
+  }
+#pragma unroll
+  for (int m = 0; m < 5; ++m) cw2[m] = r2 == 0 ? cpar<T>(cp.c2[0][m], cp.c2f[0][m]) : cpar<T>(cp.c2[1][m], cp.c2f[1][m]);
   for (int gz = zb; gz < ze; ++gz) {
     store_plane(slot_of(gz + CH));  // plane gz+2, loaded during the previous iteration
     __syncthreads();
@@ -901,17 +895,17 @@ __global__ void __launch_bounds__(CX * CWY) k_central_wall(BlockK b, CentralPara
       return acc;
     };
     auto D1 = [&](int f, int s, T inv) -> T {
-      if (WALL && s == sy && wr1 >= 0) return Y1(f, 0, 0) * inv;
+      if (s == sy && wr1 >= 0) return Y1(f, 0, 0) * inv;
       return d1w<T>(F(f, -2 * s), F(f, -s), F(f, s), F(f, 2 * s)) * inv;
     };
     auto D2 = [&](int f, int s, T inv) -> T {
-      if (WALL && s == sy && wr2 >= 0) return Y2(f) * inv;
+      if (s == sy && wr2 >= 0) return Y2(f) * inv;
       return d2w<T>(F(f, -2 * s), F(f, -s), F(f, 0), F(f, s), F(f, 2 * s)) * inv;
     };
-    // mixed derivative: central-4 along sb of the central-4 derivative along sa (WALL: the
+    // mixed derivative: central-4 along sb of the central-4 derivative along sa (the
     // closures where sa or sb is y; moving along sb keeps the point's row along sa)
     auto DM = [&](int f, int sa, int sb, T ia, T ib) -> T {
-      if (WALL && sb == sy && wr1 >= 0) {  // closure along y of the x (sa) derivatives
+      if (sb == sy && wr1 >= 0) {  // closure along y of the x (sa) derivatives
         auto dx = [&](int dy) -> T {
           const int o = dy * sy;
           return d1w<T>(Fp(f, 0, o - 2 * sa), Fp(f, 0, o - sa), Fp(f, 0, o + sa), Fp(f, 0, o + 2 * sa)) * ia;
@@ -926,7 +920,7 @@ __global__ void __launch_bounds__(CX * CWY) k_central_wall(BlockK b, CentralPara
         }
         return r * ib;
       }
-      if (WALL && sa == sy && wr1 >= 0) {  // central along sb (z) of the closure y derivatives
+      if (sa == sy && wr1 >= 0) {  // central along sb (z) of the closure y derivatives
         const int k = sb / sz;
         return d1w<T>(Y1(f, -2 * k, 0) * ia, Y1(f, -k, 0) * ia, Y1(f, k, 0) * ia, Y1(f, 2 * k, 0) * ia) * ib;
       }
@@ -972,18 +966,14 @@ __global__ void __launch_bounds__(CX * CWY) k_central_wall(BlockK b, CentralPara
         dT[j] = D1(Fd::TT, S[j], ID[j]);
         lapT += D2(Fd::TT, S[j], JD[j]);
       }
-      if constexpr (WALL) lapT += dT[1] * sdy;
+      lapT += dT[1] * sdy;
 #pragma unroll
       for (int i = 0; i < 3; ++i) {
         T s = L_(0.0);
 #pragma unroll
         for (int j = 0; j < 3; ++j) s += D2(UF[i], S[j], JD[j]);
-        if constexpr (WALL) {
-          s += du[i][1] * sdy;
-          s += L_(1.0 / 3.0) * (i == 1 ? D2(UF[i], S[i], JD[i]) + du[1][1] * sdy : D2(UF[i], S[i], JD[i]));
-        } else {
-          s += L_(1.0 / 3.0) * D2(UF[i], S[i], JD[i]);
-        }
+        s += du[i][1] * sdy;
+        s += L_(1.0 / 3.0) * (i == 1 ? D2(UF[i], S[i], JD[i]) + du[1][1] * sdy : D2(UF[i], S[i], JD[i]));
 #pragma unroll
         for (int j = 0; j < 3; ++j) {
           if (j == i) continue;

@@ -832,7 +832,9 @@ int residual(osb_ctx* c, Block& bl) {
 
 
 // Interface faces of every block: the interior of each face (full = 0) or the face with its
-// transverse halos (full = 1).
+// transverse halos (full = 1), then one direction per launch: a launch writes halos along its
+// direction and reads points inside along it, so none reads what another thread writes, and an edge
+// that two interfaces share gets the higher direction's value.
 int apply_interfaces(osb_ctx* c, int full, int fields) {
   IfBatch batch{};
   auto flush = [&]() {
@@ -844,12 +846,12 @@ int apply_interfaces(osb_ctx* c, int full, int fields) {
     batch.nfaces = 0;
     batch.total = 0;
   };
-  for (size_t ib = 0; ib < c->blocks.size(); ++ib) {
-    Block& bl = c->blocks[ib];
-    const int nv = bl.d.ndim + 2;
-    for (int d = 0; d < bl.d.ndim; ++d)
+  for (int d = 0; d < 3; ++d) {
+    for (size_t ib = 0; ib < c->blocks.size(); ++ib) {
+      Block& bl = c->blocks[ib];
+      const int nv = bl.d.ndim + 2;
       for (int side = 0; side < 2; ++side) {
-        if (bl.d.bc[d][side] != OSB_BC_INTERFACE) continue;
+        if (d >= bl.d.ndim || bl.d.bc[d][side] != OSB_BC_INTERFACE) continue;
         const osb_interface& f = bl.d.iface[d][side];
         if (f.block < 0 || f.block >= (int)c->blocks.size())
           return fail(OSB_EINVAL, "interface of block %zu dir %d side %d names block %d of %zu", ib, d, side, f.block,
@@ -899,6 +901,8 @@ int apply_interfaces(osb_ctx* c, int full, int fields) {
         batch.total += (int)total;
         if (++batch.nfaces == kIfMax || batch.total > (1 << 30)) flush();
       }
+    }
+    if (full) flush();
   }
   flush();
   return OSB_OK;

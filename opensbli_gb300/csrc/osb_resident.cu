@@ -173,6 +173,9 @@ __global__ void __launch_bounds__(RT) k_resident_1d(const Resident1D* __restrict
   const bool end[2] = {rank == 0, rank == C - 1};
   const int peer[2] = {rank > 0 ? rank - 1 : C - 1, rank < C - 1 ? rank + 1 : 0};
   const bool linked[2] = {!end[0] || per, !end[1] || per};
+  // halo points that an exchange fills (a periodic face fills the other side's); those beyond the depth of
+  // a block's end keep the caller's values
+  const int fill[2] = {end[0] ? r.depth[per ? 1 : 0] : RH, end[1] ? r.depth[per ? 0 : 1] : RH};
   auto hal = [&](int parity, int side, int m, int v) { return ((parity * 2 + side) * RH + m) * 3 + v; };
   // halo point m = 0 .. RH - 1 counted outwards from the end
   for (int u = threadIdx.x; u < 3 * n; u += blockDim.x) {
@@ -211,7 +214,8 @@ __global__ void __launch_bounds__(RT) k_resident_1d(const Resident1D* __restrict
         for (int v = 0; v < 3; ++v) {
           const double* f = L.q + v * most;
           double x;
-          if (i < 0) x = linked[0] ? L.halo[hal(parity, 0, -1 - i, v)] : halo_point(r.bc[0], f, 1, -i);
+          if (-i > fill[0] || i - n >= fill[1]) x = r.k.q[v][off + g0 + i];
+          else if (i < 0) x = linked[0] ? L.halo[hal(parity, 0, -1 - i, v)] : halo_point(r.bc[0], f, 1, -i);
           else if (i >= n) x = linked[1] ? L.halo[hal(parity, 1, i - n, v)] : halo_point(r.bc[1], f + n - 1, -1, i - n + 1);
           else if (i == 0 && !linked[0]) L.q[v * most] = x = end_point(r.bc[0], f, 1);
           else if (i == n - 1 && !linked[1]) L.q[v * most + i] = x = end_point(r.bc[1], f + i, -1);
